@@ -172,7 +172,7 @@ struct gcc_engine {
     uint64_t ver_units = 0;
     // ordering passes
     uint32_t *acc_key[2] = {nullptr, nullptr}, *acc_val[2] = {nullptr, nullptr};
-    uint32_t *op_row = nullptr, *op_pos = nullptr, *order = nullptr, *tx_rank = nullptr;
+    uint32_t *op_row = nullptr, *op_wait = nullptr, *order = nullptr, *tx_rank = nullptr;
     uint32_t *sort_counts = nullptr;
     uint64_t acc_cap = 0, counts_cap = 0, order_cap = 0;
     std::vector<uint32_t *> scan_tmp;
@@ -251,7 +251,7 @@ gcc_engine::~gcc_engine() {
     if (dev >= 0) cudaSetDevice(dev);
     void *bufs[] = {table, hash_slots, sorted, txs, meta, latch, turn, digest, commit_hi,
                     commit_lo, tx_aborts, read_log, scratch, ver_ts, ver_prev, ver_data,
-                    acc_key[0], acc_key[1], acc_val[0], acc_val[1], op_row, op_pos, order,
+                    acc_key[0], acc_key[1], acc_val[0], acc_val[1], op_row, op_wait, order,
                     tx_rank, sort_counts, ctr, tx_off_d, reqs_d, queue_tail, stamps};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -363,13 +363,13 @@ int gcc_engine::ensure_access(uint64_t n_acc) {
         if ((rc = alloc(&acc_val[j], n_acc * 4))) return rc;
     }
     if ((rc = alloc(&op_row, n_acc * 4))) return rc;
-    if ((rc = alloc(&op_pos, n_acc * 4))) return rc;
+    if ((rc = alloc(&op_wait, n_acc * 4))) return rc;
     acc_cap = n_acc;
     return GCC_OK;
 }
 
 // Access list of positions [p.batch_st, p.batch_st + n_pos) in p.order order:
-// stable sort by row, then per-access positions and each row's first turn.
+// stable sort by row, then the turn each access waits for and each row's first.
 int gcc_engine::order_pass(const KParams &p, uint64_t n_pos, int) {
     uint64_t n_acc = n_pos * kMaxOps;
     int rc = ensure_access(n_acc);
@@ -383,8 +383,8 @@ int gcc_engine::order_pass(const KParams &p, uint64_t n_pos, int) {
     kernel_launches += 1;
     uint32_t *k = acc_key[0], *v = acc_val[0];
     if ((rc = radix_sort(n_acc, rbits, &k, &v))) return rc;
-    k_access_positions<<<grid1d(n_acc, 256), 256, 0, stream>>>(k, v, n_acc, invalid, op_pos,
-                                                                turn);
+    k_access_waits<<<grid1d(n_acc, kWaitTile), kWaitThreads, 0, stream>>>(k, v, n_acc, invalid,
+                                                                          op_wait, turn);
     CK(cudaGetLastError());
     kernel_launches += 1;
     return GCC_OK;
@@ -413,7 +413,7 @@ int gcc_engine::gputx_rank(const KParams &p0) {
     if ((rc = radix_sort(n_acc, rbits, &k, &v))) return rc;
     // flags -> inclusive scan -> per-row base -> per-tx max rank
     uint32_t *f = (k == acc_key[0]) ? acc_key[1] : acc_key[0];
-    uint32_t *S = op_pos;  // free until the second ordering pass
+    uint32_t *S = op_wait;  // free until the second ordering pass
     k_rank_flags<<<grid1d(n_acc, 256), 256, 0, stream>>>(k, v, n_acc, invalid, f);
     CK(cudaGetLastError());
     if ((rc = scan(f, S, n_acc, true))) return rc;
@@ -769,12 +769,12 @@ int gcc_run(gcc_engine *e, const gcc_run_params *rp, gcc_result *out) {
         if (s == S_GACCO) {
             if ((rc = e->order_pass(p, bn, 0))) return rc;
             p.op_row = e->op_row;
-            p.op_pos = e->op_pos;
+            p.op_wait = e->op_wait;
         } else if (gputx) {
             // second pass: accesses in (rank, tx) order
             if ((rc = e->order_pass(p, bn, 0))) return rc;
             p.op_row = e->op_row;
-            p.op_pos = e->op_pos;
+            p.op_wait = e->op_wait;
         }
         CKR(cudaEventRecord(e1, st));
         uint64_t want = (bn * (uint64_t)G + block - 1) / block;
@@ -1335,7 +1335,7 @@ int gcc_run_checked(gcc_engine *e, const gcc_run_params *rp, gcc_result *out, in
             q.scratch = rp->write_mode == GCC_WRITE_ROWCOPY ? e->scratch : nullptr;
             if (ce == cudaSuccess && rc == GCC_OK) rc = e->order_pass(q, n, 0);
             q.op_row = e->op_row;
-            q.op_pos = e->op_pos;
+            q.op_wait = e->op_wait;
             if (ce == cudaSuccess && rc == GCC_OK) {
                 const int block = 256;
                 int occ = scheme_occupancy(S_GACCO, 32, block);

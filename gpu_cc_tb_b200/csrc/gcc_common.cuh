@@ -153,14 +153,14 @@ struct KParams {
     // CC metadata
     unsigned long long *meta;   // one packed word per row
     unsigned int *latch;        // per-row latch (slow_* schemes)
-    unsigned int *turn;         // per-row turn (gacco/gputx) / mvcc chain head
+    unsigned int *turn;         // per-row count of accesses done (gacco/gputx) / mvcc chain head
     // MVCC version store: one node per (batch position, op)
     unsigned long long *ver_ts;   // old version word
     unsigned int *ver_prev;       // previous node or kNoRow
     uint64_t *ver_data;           // old row image (wslot words per node)
     // precomputed per access (ordered schemes): access = pos * 16 + op
     const uint32_t *op_row;
-    const uint32_t *op_pos;
+    const uint32_t *op_wait;
     // outputs, indexed by tx id
     unsigned long long *digest;
     unsigned long long *commit_hi;
@@ -240,8 +240,8 @@ GCC_D unsigned ld_acquire(const unsigned *p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
     return r;
 }
-GCC_D void st_release(unsigned *p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
+GCC_D void red_add_rel(unsigned *p, unsigned v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
 GCC_D void set_error(Counters *c, int code, unsigned where) {

@@ -249,16 +249,87 @@ __global__ void k_access_build(KParams p, uint64_t n_pos, uint32_t invalid_key, 
     op_row[a] = row;
 }
 
-// After the stable sort by row: op_pos[a] = sorted position; the first
-// position of each row's run becomes that row's initial turn.
-__global__ void k_access_positions(const uint32_t *skeys, const uint32_t *svals, uint64_t n_acc,
-                                   uint32_t invalid_key, uint32_t *op_pos, unsigned *turn) {
-    uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (q >= n_acc) return;
-    uint32_t row = skeys[q];
-    if (row == invalid_key) return;
-    op_pos[svals[q] & 0x7FFFFFFFu] = (uint32_t)q;
-    if (q == 0 || skeys[q - 1] != row) turn[row] = (uint32_t)q;
+// After the stable sort by row, position q is the q-th access of the whole
+// list and each row's accesses are consecutive; a row's turn word starts at
+// its first position and counts up with every access done. op_wait[a] = the
+// turn that access a waits for: its own position for a write (all earlier
+// accesses of the row done), the position after the row's last earlier write
+// for a read (the row's first position if there is none), i.e. an inclusive
+// running maximum of {write: q + 1, first of its row: q, else 0}. A row's
+// first position is larger than every mark before it, so the maximum needs
+// no reset at row borders. Blocks are independent: a block whose first access
+// continues a row looks backwards for the last mark, block-wide, 1,024
+// accesses a step (one step unless a run of reads is longer than that).
+constexpr int kWaitThreads = 256;
+constexpr int kWaitTile = kWaitThreads * 4;
+
+__device__ __forceinline__ uint32_t wait_mark(const uint32_t *skeys, const uint32_t *svals,
+                                              uint64_t q) {
+    if (!(svals[q] >> 31)) return (uint32_t)q + 1u;
+    return (q == 0 || skeys[q - 1] != skeys[q]) ? (uint32_t)q : 0u;
+}
+
+__global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *skeys,
+                                                               const uint32_t *svals,
+                                                               uint64_t n_acc,
+                                                               uint32_t invalid_key,
+                                                               uint32_t *op_wait, unsigned *turn) {
+    __shared__ uint32_t s_warp[kWaitThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)blockIdx.x * kWaitTile;
+    const uint64_t q0 = base + 4ull * threadIdx.x;
+    uint32_t key[4], val[4], m[4];
+    uint32_t run = 0;
+    uint32_t before = q0 > 0 && q0 <= n_acc ? skeys[q0 - 1] : 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t q = q0 + j;
+        key[j] = q < n_acc ? skeys[q] : invalid_key;
+        val[j] = q < n_acc ? svals[q] : 0u;
+        uint32_t v = 0;
+        if (q < n_acc) {
+            const bool first = q == 0 || before != key[j];
+            if (first && key[j] != invalid_key) turn[key[j]] = (uint32_t)q;
+            v = (val[j] >> 31) ? (first ? (uint32_t)q : 0u) : (uint32_t)q + 1u;
+        }
+        before = key[j];
+        run = max(run, v);
+        m[j] = run;
+    }
+    // exclusive block-wide running maximum of the threads' maxima
+    uint32_t x = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) x = max(x, __shfl_up_sync(0xFFFFFFFFu, x, o));
+    if (lane == 31) s_warp[wid] = x;
+    uint32_t carry = __shfl_up_sync(0xFFFFFFFFu, x, 1);
+    if (lane == 0) carry = 0;
+    __syncthreads();
+    for (int w = 0; w < wid; ++w) carry = max(carry, s_warp[w]);
+    // the last mark before the block, where the block starts inside a row
+    if (base > 0 && base < n_acc && skeys[base - 1] == skeys[base] && skeys[base] != invalid_key) {
+        uint32_t found = 0;
+        for (uint64_t hi = base; hi > 0 && !found;) {
+            __syncthreads();
+            uint32_t v = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t back = 1ull + threadIdx.x + (uint64_t)j * kWaitThreads;
+                if (back <= hi) v = max(v, wait_mark(skeys, svals, hi - back));
+            }
+            v = __reduce_max_sync(0xFFFFFFFFu, v);
+            if (lane == 0) s_warp[wid] = v;
+            __syncthreads();
+            for (int w = 0; w < kWaitThreads / 32; ++w) found = max(found, s_warp[w]);
+            hi = hi > (uint64_t)kWaitTile ? hi - kWaitTile : 0ull;
+        }
+        carry = max(carry, found);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t q = q0 + j;
+        if (q < n_acc && key[j] != invalid_key)
+            op_wait[val[j] & 0x7FFFFFFFu] = (val[j] >> 31) ? max(m[j], carry) : (uint32_t)q;
+    }
 }
 
 // GPUTx: f[q] = 1 where a run continues and the pair (q-1, q) is not
