@@ -28,6 +28,7 @@
 // version-store stride, GPUTx same-rank conflicts).
 #pragma once
 #include <cooperative_groups.h>
+#include <type_traits>
 #include "gcc_common.cuh"
 
 namespace gcc {
@@ -80,6 +81,7 @@ struct Group {
         }
         return v;
     }
+    GCC_D uint32_t orv(uint32_t v) const { return __reduce_or_sync(mask, v); }
     GCC_D unsigned long long orv(unsigned long long v) const {
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) v |= __shfl_xor_sync(mask, v, o, G);
@@ -98,8 +100,13 @@ struct TxOps {
     uint32_t n;                // requests in the transaction
     uint32_t valid;            // bit k: op k exists
     uint32_t isread;           // bit k: op k reads
-    unsigned long long readmask;  // group-wide: bit i set if op i reads
+    using Mask = std::conditional_t<(MO > 32), unsigned long long, uint32_t>;
+    Mask readmask;             // group-wide: bit i set if op i reads
     uint32_t row[K];
+    // one request a lane: the field and value its write stores (FIELD mode),
+    // computed before the attempt so that no row is held for it
+    uint32_t wfield;
+    unsigned long long wval;
     // 1 + the request that failed in the last aborted 2PL / TO attempt (0:
     // none); the next one-at-a-time attempt visits it after the others
     // (unless GCC_F_REQUEST_ORDER)
@@ -120,23 +127,58 @@ constexpr int kMaxChunks = 7;  // 16-byte chunks cover up to 14 words (112 B)
 GCC_D size_t slot_of(const KParams &p, uint64_t unit, uint32_t i) {
     return ((size_t)unit * p.slot_ops + i) * p.wslot;
 }
-// Stream a row image from `src` (16-byte L2 loads), folding its words into
-// the digest term `dt` of op i and copying it to the rowcopy scratch slot and
-// the read log when those exist. Nothing is held in registers beyond one
-// chunk, so the transaction kernel fits 64 registers.
+// Read a row image from `src` (L2 loads), folding its words into the digest
+// term `dt` of op i and copying it to the rowcopy scratch slot and the read
+// log when those exist. Where a lane has one or two requests (K), loads of an
+// image are issued together before the first is used: chunk by chunk each
+// one's L2 round trip came after the one before. Rows of 11 words on 32-byte
+// boundaries (the u64 layout) are three 32-byte loads, i.e. one L2 request per
+// sector; others move in 16-byte chunks, four together with one request a
+// lane. Lanes with more requests have no registers left for that (64 with
+// 1,024-thread CTAs) and go chunk by chunk. Measured: see ycsb_kernel.
+template <int K>
 GCC_D void read_image(const KParams &p, const uint64_t *src, uint32_t tx, uint64_t pos,
                       uint32_t i, unsigned long long &dt) {
-    const ulonglong2 *s = (const ulonglong2 *)src;
     ulonglong2 *sc = p.scratch ? (ulonglong2 *)(p.scratch + slot_of(p, pos, i)) : nullptr;
     ulonglong2 *lg = p.read_log ? (ulonglong2 *)(p.read_log + slot_of(p, tx, i)) : nullptr;
+    auto keep = [&](int c, unsigned long long x, unsigned long long y) {
+        if (sc) __stcg(sc + c, make_ulonglong2(x, y));
+        if (lg) __stcg(lg + c, make_ulonglong2(x, y));
+    };
+    // the digest's terms, each word's tag counted up
+    unsigned long long tag = (unsigned long long)(i * 16u + 1u) * kDigestStep;
+    auto fold = [&](unsigned long long w) {
+        dt += splitmix64(w ^ tag);
+        tag += kDigestStep;
+    };
+    if (K <= 2 && p.wide) {
+        Sector s[3];
 #pragma unroll
-    for (int c = 0; c < kMaxChunks; ++c) {
-        if (2 * c < (int)p.words) {
-            ulonglong2 v = __ldcg(s + c);
-            dt += digest_term(v.x, i, 2u * c);
-            if (2 * c + 1 < (int)p.words) dt += digest_term(v.y, i, 2u * c + 1u);
-            if (sc) __stcg(sc + c, v);
-            if (lg) __stcg(lg + c, v);
+        for (int c = 0; c < 3; ++c) s[c] = ld_cg32(src + 4 * c);
+#pragma unroll
+        for (int k = 0; k < 11; ++k) fold(s[k / 4].w[k % 4]);
+        if (sc || lg) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) keep(c, s[c / 2].w[c % 2 * 2], s[c / 2].w[c % 2 * 2 + 1]);
+        }
+        return;
+    }
+    constexpr int kTogether = K == 1 ? 4 : 1;
+    const ulonglong2 *s = (const ulonglong2 *)src;
+#pragma unroll
+    for (int h = 0; h < kMaxChunks; h += kTogether) {
+        ulonglong2 v[kTogether];
+#pragma unroll
+        for (int j = 0; j < kTogether; ++j)
+            if (h + j < kMaxChunks && 2 * (h + j) < (int)p.words) v[j] = __ldcg(s + h + j);
+#pragma unroll
+        for (int j = 0; j < kTogether; ++j) {
+            const int c = h + j;
+            if (c < kMaxChunks && 2 * c < (int)p.words) {
+                fold(v[j].x);
+                if (2 * c + 1 < (int)p.words) fold(v[j].y);
+                keep(c, v[j].x, v[j].y);
+            }
         }
     }
 }
@@ -175,7 +217,7 @@ GCC_D unsigned long long apply_ext(const KParams &p, uint64_t *r, uint32_t tx, u
         return 0ull;
     }
     unsigned long long dt = 0;
-    read_image(p, r, tx, 0, i, dt);
+    read_image<4>(p, r, tx, 0, i, dt);
     unsigned long long *fw = (unsigned long long *)(r + 1 + f);
     const unsigned long long a = __ldcg(fw);
     if (op == GCC_OP_ADD) {
@@ -199,11 +241,11 @@ GCC_D unsigned long long apply_ext(const KParams &p, uint64_t *r, uint32_t tx, u
 // Apply write op i of tx to `row` (GCC_WRITE_FIELD or GCC_WRITE_ROWCOPY, or
 // an extended op when the run enables them). Extended ops exist only in the
 // variable-length kernels (EXT): the 16-request kernels keep their registers.
-template <bool EXT>
-GCC_D void apply_write(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos,
-                       uint32_t i, unsigned long long readmask, unsigned long long &dg) {
+template <class TX>
+GCC_D void apply_write(const KParams &p, const TX &s, uint32_t row, uint32_t tx, uint64_t pos,
+                       uint32_t i, unsigned long long &dg) {
     uint64_t *r = row_ptr(p, row);
-    if (EXT && p.ext_ops) {
+    if (TX::kExt && p.ext_ops) {
         const int32_t w = p.txs ? __ldg(&p.txs[tx].requests[i].read)
                                 : __ldg(&p.reqs[p.tx_off[tx] + i].read);
         if (w < 0) {
@@ -212,12 +254,12 @@ GCC_D void apply_write(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos
         }
     }
     if (p.write_mode == GCC_WRITE_FIELD) {
-        uint32_t f = write_field(p.write_seed, tx, i);
-        __stcg((unsigned long long *)(r + 1 + f),
-               (unsigned long long)write_value(p.write_seed, tx, i));
+        const uint32_t f = TX::K == 1 ? s.wfield : write_field(p.write_seed, tx, i);
+        const unsigned long long v = TX::K == 1 ? s.wval : write_value(p.write_seed, tx, i);
+        __stcg((unsigned long long *)(r + 1 + f), v);
         return;
     }
-    int src = rowcopy_src(readmask, i);
+    int src = rowcopy_src(s.readmask, i);
     if (src < 0) {
 #pragma unroll
         for (int c = 0; c < kMaxChunks; ++c)
@@ -284,59 +326,96 @@ GCC_D unsigned long long alloc_ts(Counters *c) {
 
 // Per-attempt leader-side timing accumulators.
 struct Clocks {
-    unsigned long long ts, wait, mng;
+    unsigned long long ts, wait;
 };
+
+// An attempt works through its requests in stages: the group tries every
+// request of a stage's mask (bit k: the lane's k-th) until all are done, one
+// fails, or the bounded wait runs out. All stages of an attempt go through one
+// inlined copy of `op(k)`, which returns an OpResult.
+enum OpResult : int { O_DONE = 0, O_FAIL = 1, O_RETRY = 2, O_ERR = 3 };
+struct Waiting {
+    bool any = false;
+    uint64_t t0 = 0;   // first wait of the attempt
+    long long clk = 0;
+};
+template <int G, int K, class OP>
+GCC_D int run_stage(const KParams &p, const Group<G> &g, uint32_t pending, Waiting &w, unsigned site,
+                    OP op) {
+    while (true) {
+        uint32_t st = 0;  // 1: pending, 2: failed, 4: error
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (!((pending >> k) & 1u) || (st & 6u)) continue;
+            const int r = op(k);
+            if (r == O_DONE) pending &= ~(1u << k);
+            else if (r == O_FAIL) st |= 2u;
+            else if (r == O_ERR) st |= 4u;
+        }
+        if (pending) st |= 1u;
+        st = g.orv(st);
+        if (st & 4u) return O_ERR;
+        if (st & 2u) return O_FAIL;
+        if (!st) return O_DONE;
+        if (!w.any) { w.any = true; w.t0 = gtimer(); w.clk = clock64(); }
+        wait_pause();
+        if (g.any(expired(w.t0, p.spin_limit_ns) || error_raised(p.ctr))) {
+            if (g.glane == 0) set_error(p.ctr, GCC_ETIMEOUT, site);
+            return O_ERR;
+        }
+    }
+}
+// The stage of request i alone.
+template <int G>
+GCC_D uint32_t only(const Group<G> &g, uint32_t i) {
+    return g.glane == (int)(i % G) ? 1u << (i / G) : 0u;
+}
 
 // ===========================================================================
 // 2PL no-wait / wait-die (twopl.cuh:233-322; slow_twopl.cuh:238-331)
 // ===========================================================================
-enum LockResult : int { L_OK = 0, L_DIE = 1, L_WAIT = 2, L_ERR = 3 };
-
-template <bool WD>
-GCC_D int tpl_shared(const KParams &p, uint32_t row, uint32_t tx) {
+// One request of the fast variants: a speculative reader increment, or the
+// exclusive word into a free one. `again`: the request waited already, so a
+// reader looks before it increments. (With several requests a lane (K) the
+// branch-free form costs more in spilled registers than it saves.)
+template <bool WD, int K>
+GCC_D int tpl_request(const KParams &p, uint32_t row, uint32_t tx, bool rd, bool again) {
     unsigned long long *m = p.meta + row;
-    if (WD) {
-        unsigned long long w = ld_cg(m);
-        if (w & tpl::kExcl) return tpl::holder(w) < tx ? L_DIE : L_WAIT;
+    if (WD && again && rd) {
+        const unsigned long long w = ld_cg(m);
+        if (w & tpl::kExcl) return tpl::holder(w) < tx ? O_FAIL : O_RETRY;
     }
-    unsigned long long old = atom_add_acq(m, 1ull);
-    if (!(old & tpl::kExcl)) return L_OK;
-    atomicAdd(m, ~0ull);  // undo the speculative reader increment
-    if (!WD) return L_DIE;
-    return tpl::holder(old) < tx ? L_DIE : L_WAIT;
-}
-template <bool WD>
-GCC_D int tpl_excl(const KParams &p, uint32_t row, uint32_t tx) {
-    unsigned long long old = atom_cas_acq(p.meta + row, 0ull, tpl::excl_word(tx));
-    if (old == 0ull) return L_OK;
-    if (!WD) return L_DIE;
-    if (!(old & tpl::kExcl)) return L_DIE;  // shared holders: requester dies
-    return tpl::holder(old) < tx ? L_DIE : L_WAIT;
+    const unsigned long long old = atom_lock_acq<(K == 1)>(m, rd, tpl::excl_word(tx));
+    if (rd ? !(old & tpl::kExcl) : old == 0ull) return O_DONE;
+    if (rd) atomicAdd(m, ~0ull);  // undo the speculative reader increment
+    if (!WD || !(old & tpl::kExcl)) return O_FAIL;  // (shared holders: a writer dies)
+    return tpl::holder(old) < tx ? O_FAIL : O_RETRY;
 }
 // Latch variants: plain read/modify/write of the same word under a latch.
 template <bool WD>
 GCC_D int slow_tpl_lock(const KParams &p, uint32_t row, uint32_t tx, bool shared) {
-    if (!latch_acquire(p, row)) return L_ERR;
+    if (!latch_acquire(p, row)) return O_ERR;
     volatile unsigned long long *m = p.meta + row;
     unsigned long long w = *m;
     int r;
     if (shared) {
-        if (!(w & tpl::kExcl)) { *m = w + 1ull; r = L_OK; }
-        else r = (!WD || tpl::holder(w) < tx) ? L_DIE : L_WAIT;
+        if (!(w & tpl::kExcl)) { *m = w + 1ull; r = O_DONE; }
+        else r = (!WD || tpl::holder(w) < tx) ? O_FAIL : O_RETRY;
     } else {
-        if (w == 0ull) { *m = tpl::excl_word(tx); r = L_OK; }
-        else if (!WD || !(w & tpl::kExcl)) r = L_DIE;
-        else r = tpl::holder(w) < tx ? L_DIE : L_WAIT;
+        if (w == 0ull) { *m = tpl::excl_word(tx); r = O_DONE; }
+        else if (!WD || !(w & tpl::kExcl)) r = O_FAIL;
+        else r = tpl::holder(w) < tx ? O_FAIL : O_RETRY;
     }
     latch_release(p, row);
     return r;
 }
+// The fast variants' releases are plain reductions: the caller has fenced
+// (once for all lanes) where rows were read or written under the locks.
 template <bool SLOW>
 GCC_D bool tpl_unlock(const KParams &p, uint32_t row, bool shared) {
     if (!SLOW) {
-        // release: this lane's reads / writes of the row come before
-        if (shared) red_add_rel(p.meta + row, ~0ull);
-        else red_and_rel(p.meta + row, tpl::kReaders);
+        if (shared) atomicAdd(p.meta + row, ~0ull);
+        else atomicAnd(p.meta + row, tpl::kReaders);
         return true;
     }
     if (shared) {
@@ -353,10 +432,9 @@ GCC_D bool tpl_unlock(const KParams &p, uint32_t row, bool shared) {
     return true;
 }
 
-template <bool WD, bool SLOW>
-GCC_D int tpl_lock(const KParams &p, uint32_t row, uint32_t tx, bool rd) {
-    return SLOW ? slow_tpl_lock<WD>(p, row, tx, rd)
-                : (rd ? tpl_shared<WD>(p, row, tx) : tpl_excl<WD>(p, row, tx));
+template <bool WD, bool SLOW, int K>
+GCC_D int tpl_lock(const KParams &p, uint32_t row, uint32_t tx, bool rd, bool again) {
+    return SLOW ? slow_tpl_lock<WD>(p, row, tx, rd) : tpl_request<WD, K>(p, row, tx, rd, again);
 }
 
 // First attempts take all locks at once (one ballot decides); after
@@ -382,13 +460,10 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
                       uint64_t pos, unsigned long long &dg, Clocks &ck, bool ordered) {
     constexpr int K = TX::K;
     uint32_t held = 0;
-    bool fail = false, err = false;
     uint32_t obst = kNoRow;         // row whose lock request failed
     bool obst_x = false;            // ... and whether it was an exclusive request
     uint32_t obst_i = 0xFFFFFFFFu;  // ... and its request index
-    uint64_t t0 = gtimer();
-    long long cw = clock64();
-    bool first = true;
+    Waiting w;
     // planned: this attempt locks the requests outside the plan at once, then
     // the plan's requests in plan order; late bit k: op glane + k * G is planned
     bool planned = false;
@@ -410,78 +485,31 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
                 if ((plan_mask(pl) >> (g.glane + k * G)) & 1u) late |= 1u << k;
         }
     }
-    uint32_t pending = s.valid & ~late;
-    // every pending request at once; a conflict fails the attempt (no-wait)
-    // or, under wait-die, a younger holder makes the request wait
-    auto lock_at_once = [&]() {
-        while (true) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (!((pending >> k) & 1u) || fail || err) continue;
-                int r = tpl_lock<WD, SLOW>(p, s.row[k], tx, (s.isread >> k) & 1u);
-                if (r == L_OK) { held |= 1u << k; pending &= ~(1u << k); }
-                else if (r == L_DIE) {
-                    fail = true;
-                    obst = s.row[k];
-                    obst_x = !((s.isread >> k) & 1u);
-                    obst_i = (uint32_t)(g.glane + k * G);
-                }
-                else if (r == L_ERR) err = true;
+    // Stages: the requests that go at once, then (ordered) one after another,
+    // then whatever a plan did not list, as a plan only orders. A conflict
+    // fails the attempt (no-wait) or, under wait-die, a younger holder makes
+    // the request wait.
+    uint32_t pending = ordered && !planned ? 0u : s.valid & ~late;
+    const uint32_t n_seq = !ordered ? 0u : planned ? plan_count(pl) : s.n;
+    int r = O_DONE;
+    for (uint32_t j = 0;; ++j) {
+        r = run_stage<G, K>(p, g, pending, w, W_TPL_WD, [&](int k) -> int {
+            const bool rd = (s.isread >> k) & 1u;
+            const int q = tpl_lock<WD, SLOW, K>(p, s.row[k], tx, rd, w.any);
+            if (q == O_DONE) held |= 1u << k;
+            else if (q == O_FAIL) {
+                obst = s.row[k];
+                obst_x = !rd;
+                obst_i = (uint32_t)(g.glane + k * G);
             }
-            bool gf = g.any(fail), ge = g.any(err), gp = g.any(pending != 0u);
-            if (ge) { fail = true; err = true; break; }
-            if (gf || !gp) { fail = gf; break; }
-            if (first) { first = false; cw = clock64(); }
-            wait_pause();
-            if (g.any(expired(t0, p.spin_limit_ns) || error_raised(p.ctr))) {
-                if (g.glane == 0) set_error(p.ctr, GCC_ETIMEOUT, W_TPL_WD);
-                fail = true; err = true; break;
-            }
-        }
-    };
-    if (ordered) {
-        if (planned) lock_at_once();  // the requests outside the plan
-        const uint32_t n_seq = planned ? plan_count(pl) : s.n;
-        for (uint32_t j = 0; j < n_seq && !fail; ++j) {
-            const uint32_t i = planned ? plan_op(pl, j) : j;
-            const int owner = (int)(i % G), kk = (int)(i / G);
-            int r = L_OK;
-            if (g.glane == owner) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (k != kk || !((s.valid >> k) & 1u) || ((held >> k) & 1u)) continue;
-                    while (true) {
-                        r = tpl_lock<WD, SLOW>(p, s.row[k], tx, (s.isread >> k) & 1u);
-                        if (r != L_WAIT) break;
-                        if (first) { first = false; cw = clock64(); }
-                        wait_pause();
-                        if (expired(t0, p.spin_limit_ns) || error_raised(p.ctr)) {
-                            set_error(p.ctr, GCC_ETIMEOUT, W_TPL_WD);
-                            r = L_ERR;
-                            break;
-                        }
-                    }
-                    if (r == L_OK) held |= 1u << k;
-                    else if (r == L_DIE) {
-                        obst = s.row[k];
-                        obst_x = !((s.isread >> k) & 1u);
-                        obst_i = i;
-                    }
-                }
-            }
-            r = g.bcast(r, owner);
-            if (r == L_DIE) fail = true;
-            else if (r == L_ERR) { fail = true; err = true; }
-        }
-        // a plan only orders: whatever it did not list is locked now
-        if (planned && !fail) {
-            pending = s.valid & ~held;
-            lock_at_once();
-        }
-    } else {
-        lock_at_once();
+            return q;
+        });
+        if (r != O_DONE || j > n_seq || (j == n_seq && !planned)) break;
+        if (j < n_seq) pending = only(g, planned ? plan_op(pl, j) : j) & s.valid & ~held;
+        else pending = s.valid & ~held;
     }
-    if (!first) ck.wait += clock64() - cw;
+    if (w.any) ck.wait += clock64() - w.clk;
+    const bool fail = r != O_DONE, err = r == O_ERR;
     if (fail) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
@@ -513,16 +541,15 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         if (((s.valid & s.isread) >> k) & 1u) {
-            read_image(p, row_ptr(p, s.row[k]), tx, pos, (uint32_t)(g.glane + k * G), dg);
+            read_image<K>(p, row_ptr(p, s.row[k]), tx, pos, (uint32_t)(g.glane + k * G), dg);
         }
     }
     if (p.write_mode == GCC_WRITE_ROWCOPY) g.sync();
 #pragma unroll
     for (int k = 0; k < K; ++k)
         if (((s.valid & ~s.isread) >> k) & 1u)
-            apply_write<TX::kExt>(p, s.row[k], tx, pos, (uint32_t)(g.glane + k * G), s.readmask, dg);
-    // (the fast variants' unlocks are release operations)
-    if (SLOW) fence_acq_rel();
+            apply_write(p, s, s.row[k], tx, pos, (uint32_t)(g.glane + k * G), dg);
+    fence_acq_rel();  // the rows' reads and writes come before the releases
     bool uerr = false;
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -533,9 +560,29 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
 // ===========================================================================
 // Timestamp ordering (to.cuh:104-270; slow_to.cuh:137-238)
 // ===========================================================================
-enum OpResult : int { O_DONE = 0, O_FAIL = 1, O_RETRY = 2, O_ERR = 3 };
-
-template <bool SLOW>
+// After a row's image was read under the committed word x (wts(x) <= ts): make
+// its rts cover ts. The image is of version wts(x) as long as the word keeps
+// that wts and stays committed; another reader raising rts meanwhile does not
+// change it, so only the raise is tried again, not the read. False: a writer
+// came in.
+GCC_D bool rts_cover(unsigned long long *m, unsigned long long x, uint64_t ts) {
+    fence_acq_rel();  // the image's loads come before the look or the raise
+    const unsigned long long wts = tso::wts(x);
+    bool seen = false;  // x was read after the image
+    while (!(x & tso::kUnc) && tso::wts(x) == wts) {
+        if (tso::rts(x) >= ts) {
+            if (seen) return true;
+            x = ld_cg(m);
+        } else {
+            const unsigned long long old = atomicCAS(m, x, tso::make(false, ts, wts));
+            if (old == x) return true;
+            x = old;
+        }
+        seen = true;
+    }
+    return false;
+}
+template <bool SLOW, int K>
 GCC_D int to_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint64_t pos,
                   uint32_t i, unsigned long long &dt) {
     unsigned long long *m = p.meta + row;
@@ -546,7 +593,7 @@ GCC_D int to_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint
         if (tso::wts(x) > ts) r = O_FAIL;
         else if (x & tso::kUnc) r = O_RETRY;
         else {
-            read_image(p, row_ptr(p, row), tx, pos, i, dt);
+            read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
             uint64_t rts = tso::rts(x) > ts ? tso::rts(x) : ts;
             *(volatile unsigned long long *)m = tso::make(false, rts, tso::wts(x));
             r = O_DONE;
@@ -554,17 +601,18 @@ GCC_D int to_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint
         latch_release(p, row);
         return r;
     }
-    unsigned long long x = ld_cg(m);
+    const unsigned long long x = ld_acquire(m);
     if (tso::wts(x) > ts) return O_FAIL;
     if (x & tso::kUnc) return O_RETRY;  // wait for the older writer
-    read_image(p, row_ptr(p, row), tx, pos, i, dt);
+    read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
+    if (K == 1) return rts_cover(m, x, ts) ? O_DONE : O_RETRY;
+    // (a lane with several requests keeps the short form: a fence for each of
+    // them took wd 0 from 36 to 14 M tx/s)
     if (tso::rts(x) >= ts) {
-        // rts already covers this reader: only check the snapshot held
         fence_acq_rel();
         return ld_cg(m) == x ? O_DONE : O_RETRY;
     }
-    unsigned long long nx = tso::make(false, ts, tso::wts(x));
-    return atomicCAS(m, x, nx) == x ? O_DONE : O_RETRY;
+    return atomicCAS(m, x, tso::make(false, ts, tso::wts(x))) == x ? O_DONE : O_RETRY;
 }
 template <bool SLOW>
 GCC_D int to_write(const KParams &p, uint32_t row, uint64_t ts, unsigned long long &prev) {
@@ -602,10 +650,7 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
     }
     uint32_t wrote = 0;
     unsigned long long prev[K];
-    bool fail = false, err = false;
-    uint64_t t0 = gtimer();
-    bool first = true;
-    long long cw = 0;
+    Waiting w;
     uint32_t fail_i = 0xFFFFFFFFu;  // request index of this lane's failed op
     // A one-at-a-time retry visits every request but one at once first and
     // then the one that failed in the previous attempt, so a contended row
@@ -624,85 +669,38 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
                 if ((uint32_t)(g.glane + k * G) == late_i) late |= 1u << k;
         }
     }
-    uint32_t pending = s.valid & ~late;
-    // One request: read (waits while an older writer's version is
-    // uncommitted) or write (marks the row uncommitted with this ts).
-    auto op = [&](int k) -> int {
-        const uint32_t i = g.glane + k * G;
-        int r;
-        if ((s.isread >> k) & 1u) {
-            unsigned long long dt = 0;
-            r = to_read<SLOW>(p, s.row[k], ts, tx, pos, i, dt);
-            if (r == O_DONE) dg += dt;
-        } else {
-            r = to_write<SLOW>(p, s.row[k], ts, prev[k]);
-            if (r == O_DONE) wrote |= 1u << k;
-        }
-        if (r == O_FAIL) fail_i = i;
-        return r;
-    };
-    // every pending request at once (reads of rows an older writer holds
-    // uncommitted wait and retry)
-    auto all_at_once = [&]() {
-        while (true) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (!((pending >> k) & 1u) || fail || err) continue;
-                int r = op(k);
-                if (r == O_DONE) pending &= ~(1u << k);
-                else if (r == O_FAIL) fail = true;
-                else if (r == O_ERR) err = true;
+    // Stages: all requests at once; on ordered retries one at a time, so two
+    // writers cannot keep holding each other's rows uncommitted and aborting
+    // each other. A request reads (it waits while an older writer's version is
+    // uncommitted) or marks its row uncommitted with this ts.
+    const bool split = late_i != 0xFFFFFFFFu;
+    uint32_t pending = ordered && !split ? 0u : s.valid & ~late;
+    const uint32_t n_seq = !ordered ? 0u : split ? 1u : s.n;
+    int r = O_DONE;
+    for (uint32_t j = 0;; ++j) {
+        r = run_stage<G, K>(p, g, pending, w, W_TO_READ, [&](int k) -> int {
+            const uint32_t i = g.glane + k * G;
+            int q;
+            if ((s.isread >> k) & 1u) {
+                unsigned long long dt = 0;
+                q = to_read<SLOW, K>(p, s.row[k], ts, tx, pos, i, dt);
+                if (q == O_DONE) dg += dt;
+            } else {
+                q = to_write<SLOW>(p, s.row[k], ts, prev[k]);
+                if (q == O_DONE) wrote |= 1u << k;
             }
-            bool ge = g.any(err), gf = g.any(fail), gp = g.any(pending != 0u);
-            if (ge) { fail = err = true; break; }
-            if (gf || !gp) { fail = gf; break; }
-            if (first) { first = false; cw = clock64(); }
-            wait_pause();
-            if (g.any(expired(t0, p.spin_limit_ns) || error_raised(p.ctr))) {
-                if (g.glane == 0) set_error(p.ctr, GCC_ETIMEOUT, W_TO_READ);
-                fail = err = true; break;
-            }
-        }
-    };
-    if (ordered) {
-        // Retries visit the requests one at a time, so two writers cannot
-        // keep holding each other's rows uncommitted and aborting each other.
-        const bool split = late_i != 0xFFFFFFFFu;
-        if (split) all_at_once();  // the others
-        const uint32_t n_seq = split ? 1u : s.n;
-        for (uint32_t j = 0; j < n_seq && !fail; ++j) {
-            const uint32_t i = split ? late_i : j;
-            const int owner = (int)(i % G), kk = (int)(i / G);
-            int r = O_DONE;
-            if (g.glane == owner) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (k != kk || !((s.valid >> k) & 1u)) continue;
-                    while (true) {
-                        r = op(k);
-                        if (r != O_RETRY) break;
-                        if (first) { first = false; cw = clock64(); }
-                        wait_pause();
-                        if (expired(t0, p.spin_limit_ns) || error_raised(p.ctr)) {
-                            set_error(p.ctr, GCC_ETIMEOUT, W_TO_READ);
-                            r = O_ERR;
-                            break;
-                        }
-                    }
-                }
-            }
-            r = g.bcast(r, owner);
-            if (r == O_FAIL) fail = true;
-            else if (r == O_ERR) fail = err = true;
-        }
-    } else {
-        all_at_once();
+            if (q == O_FAIL) fail_i = i;
+            return q;
+        });
+        if (r != O_DONE || j == n_seq) break;
+        pending = only(g, split ? late_i : j) & s.valid;
     }
+    const bool fail = r != O_DONE, err = r == O_ERR;
     if (!SLOW && fail && !err && !(p.flags & GCC_F_REQUEST_ORDER)) {
         const uint32_t fi = __reduce_min_sync(g.mask, fail_i);
         s.obst_op = fi == 0xFFFFFFFFu ? 0u : fi + 1u;
     }
-    if (!first) ck.wait += clock64() - cw;
+    if (w.any) ck.wait += clock64() - w.clk;
     if (fail) {
         // restore the words this attempt marked uncommitted (to.cuh:255-270)
 #pragma unroll
@@ -719,7 +717,7 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
     if (p.write_mode == GCC_WRITE_ROWCOPY) g.sync();
 #pragma unroll
     for (int k = 0; k < K; ++k)
-        if ((wrote >> k) & 1u) apply_write<TX::kExt>(p, s.row[k], tx, pos, g.glane + k * G, s.readmask, dg);
+        if ((wrote >> k) & 1u) apply_write(p, s, s.row[k], tx, pos, g.glane + k * G, dg);
     fence_acq_rel();
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -745,39 +743,22 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
 // (mvcc.cuh:143 leaves the copy commented out) and each version owns a full
 // row image (mvcc.cuh:142 strides the version data by sizeof(version_node)).
 // ===========================================================================
-template <bool SLOW>
+template <bool SLOW, int K>
 GCC_D int mvcc_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint64_t pos,
                     uint32_t i, unsigned long long &dt) {
     unsigned long long *m = p.meta + row;
     if (SLOW && !latch_acquire(p, row)) return O_ERR;
-    unsigned long long x = SLOW ? *(volatile unsigned long long *)m : ld_cg(m);
+    const unsigned long long x = SLOW ? *(volatile unsigned long long *)m : ld_acquire(m);
     int r;
     if (x & tso::kUnc) {
         r = O_RETRY;
     } else if (tso::wts(x) <= ts) {
-        read_image(p, row_ptr(p, row), tx, pos, i, dt);
-        if (SLOW) {
+        read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
+        if (!SLOW) {
+            r = rts_cover(m, x, ts) ? O_DONE : O_RETRY;
+        } else {
             if (tso::rts(x) < ts) *(volatile unsigned long long *)m = tso::make(false, ts, tso::wts(x));
             r = O_DONE;
-        } else {
-            // The image is of version wts(x) as long as the word keeps that
-            // wts and stays committed. Another reader raising rts meanwhile
-            // does not change it, so only the raise is tried again.
-            fence_acq_rel();
-            const unsigned long long wts = tso::wts(x);
-            r = O_RETRY;
-            bool seen = false;  // x was read after the image
-            while (!(x & tso::kUnc) && tso::wts(x) == wts) {
-                if (tso::rts(x) >= ts) {
-                    if (seen) { r = O_DONE; break; }
-                    x = ld_cg(m);
-                } else {
-                    const unsigned long long old = atomicCAS(m, x, tso::make(false, ts, wts));
-                    if (old == x) { r = O_DONE; break; }
-                    x = old;
-                }
-                seen = true;
-            }
         }
     } else {
         // walk the version chain to the newest version with wts <= ts
@@ -793,7 +774,7 @@ GCC_D int mvcc_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, ui
         } else {
             // versions never change once linked, and the row's committed wts is
             // past ts already: no later write can come between
-            read_image(p, p.ver_data + (size_t)node * p.wslot, tx, pos, i, dt);
+            read_image<K>(p, p.ver_data + (size_t)node * p.wslot, tx, pos, i, dt);
             r = O_DONE;
         }
     }
@@ -818,56 +799,38 @@ GCC_D int attempt_mvcc(const KParams &p, const Group<G> &g, const TX &s, uint32_
     }
     uint32_t wrote = 0;
     unsigned long long prev[K];
-    bool fail = false, err = false, twice = false;
-    const uint64_t t0 = gtimer();
-    const long long cw = clock64();
-    // One round of the reads, or the writes, that are still pending.
-    auto step = [&](int k) -> int {
-        if ((s.isread >> k) & 1u) {
-            unsigned long long dt = 0;
-            const int r = mvcc_read<SLOW>(p, s.row[k], ts, tx, pos, (uint32_t)(g.glane + k * G), dt);
-            if (r == O_DONE) dg += dt;
-            return r;
-        }
-        const int r = to_write<SLOW>(p, s.row[k], ts, prev[k]);
-        if (r == O_DONE) {
-            wrote |= 1u << k;
-            twice |= tso::rts(prev[k]) == ts;
-        }
-        return r;
-    };
-    auto all_of = [&](uint32_t pending) {
-        while (true) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (!((pending >> k) & 1u) || fail || err) continue;
-                const int r = step(k);
-                if (r == O_DONE) pending &= ~(1u << k);
-                else if (r == O_FAIL) fail = true;
-                else if (r == O_ERR) err = true;
+    bool twice = false;
+    Waiting w;
+    // Stages: the reads, then the writes, at once or (ordered) one by one.
+    uint32_t pending = s.valid & s.isread;
+    unsigned long long todo = ~(unsigned long long)s.readmask & (s.n < 64u ? (1ull << s.n) - 1ull : ~0ull);
+    int r = O_DONE;
+    while (true) {
+        r = run_stage<G, K>(p, g, pending, w, W_MVCC_READ, [&](int k) -> int {
+            if ((s.isread >> k) & 1u) {
+                unsigned long long dt = 0;
+                const int q = mvcc_read<SLOW, K>(p, s.row[k], ts, tx, pos, (uint32_t)(g.glane + k * G), dt);
+                if (q == O_DONE) dg += dt;
+                return q;
             }
-            const bool ge = g.any(err), gf = g.any(fail), gp = g.any(pending != 0u);
-            if (ge || gf || !gp) { err = ge; fail = gf || ge; return; }
-            wait_pause();
-            if (g.any(expired(t0, p.spin_limit_ns) || error_raised(p.ctr))) {
-                if (g.glane == 0) set_error(p.ctr, GCC_ETIMEOUT, W_MVCC_READ);
-                fail = err = true;
-                return;
+            const int q = to_write<SLOW>(p, s.row[k], ts, prev[k]);
+            if (q == O_DONE) {
+                wrote |= 1u << k;
+                twice |= tso::rts(prev[k]) == ts;
             }
-        }
-    };
-    all_of(s.valid & s.isread);
-    if (!fail && !ordered) {
-        all_of(s.valid & ~s.isread);
-    } else if (!fail) {
-        unsigned long long todo = ~s.readmask & (s.n < 64u ? (1ull << s.n) - 1ull : ~0ull);
-        for (; todo && !fail; todo &= todo - 1ull) {
-            const uint32_t i = (uint32_t)(__ffsll((long long)todo) - 1);
-            const bool mine = g.glane == (int)(i % G);
-            all_of(mine ? 1u << (i / G) : 0u);
+            return q;
+        });
+        if (r != O_DONE || !todo) break;
+        if (ordered) {
+            pending = only(g, (uint32_t)(__ffsll((long long)todo) - 1));
+            todo &= todo - 1ull;
+        } else {
+            pending = s.valid & ~s.isread;
+            todo = 0;
         }
     }
-    ck.wait += clock64() - cw;
+    if (w.any) ck.wait += clock64() - w.clk;
+    bool fail = r != O_DONE, err = r == O_ERR;
     // A row that this transaction read and then marked (its own timestamp is
     // the row's rts): the read belongs before the write. A request order that
     // has the write first would have to read its own uncommitted row, which no
@@ -917,7 +880,7 @@ GCC_D int attempt_mvcc(const KParams &p, const Group<G> &g, const TX &s, uint32_
         p.ver_prev[node] = ld_cg(p.turn + row);
         fence_acq_rel();
         atomicExch(p.turn + row, node);
-        apply_write<TX::kExt>(p, row, tx, pos, i, s.readmask, dg);
+        apply_write(p, s, row, tx, pos, i, dg);
         fence_acq_rel();
         atomicExch(p.meta + row, tso::make(false, ts, ts));
     }
@@ -930,7 +893,7 @@ GCC_D int attempt_mvcc(const KParams &p, const Group<G> &g, const TX &s, uint32_
 // the write-set term from a field Write never sets (silo.cuh:306-310), which
 // lets a record's ts repeat and a stale read validate.
 // ===========================================================================
-template <bool SLOW>
+template <bool SLOW, int K>
 GCC_D int silo_read(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos, uint32_t i,
                     unsigned long long &dt, unsigned long long &ts) {
     unsigned long long *m = p.meta + row;
@@ -938,18 +901,16 @@ GCC_D int silo_read(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos, u
         if (!latch_acquire(p, row)) return O_ERR;
         unsigned long long x = *(volatile unsigned long long *)m;
         int r = O_RETRY;
-        if (!(x & silo::kLock)) { read_image(p, row_ptr(p, row), tx, pos, i, dt); ts = silo::ts(x); r = O_DONE; }
+        if (!(x & silo::kLock)) { read_image<K>(p, row_ptr(p, row), tx, pos, i, dt); ts = silo::ts(x); r = O_DONE; }
         latch_release(p, row);
         return r;
     }
-    unsigned long long x1 = ld_cg(m);
-    if (x1 & silo::kLock) return O_RETRY;
+    const unsigned long long x = ld_acquire(m);
+    if (x & silo::kLock) return O_RETRY;
+    read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
     fence_acq_rel();
-    read_image(p, row_ptr(p, row), tx, pos, i, dt);
-    fence_acq_rel();
-    unsigned long long x2 = ld_cg(m);
-    if (x1 != x2) return O_RETRY;
-    ts = silo::ts(x1);
+    if (ld_cg(m) != x) return O_RETRY;
+    ts = silo::ts(x);
     return O_DONE;
 }
 // No-wait write lock: O_DONE (cur = word before locking), O_FAIL if locked.
@@ -965,13 +926,9 @@ GCC_D int occ_lock(const KParams &p, uint32_t row, unsigned long long lockbit,
         latch_release(p, row);
         return r;
     }
-    for (int tries = 0; tries < 1 << 20; ++tries) {
-        unsigned long long x = ld_cg(m);
-        if (x & lockbit) return O_FAIL;
-        if (atomicCAS(m, x, x | lockbit) == x) { cur = x; return O_DONE; }
-    }
-    set_error(p.ctr, GCC_ETIMEOUT, W_CAS);
-    return O_ERR;
+    // one round trip: setting a set bit changes nothing
+    cur = atom_or_acq(m, lockbit);
+    return (cur & lockbit) ? O_FAIL : O_DONE;
 }
 
 // Lock the write set, no-wait (silo.cuh:268-281, tictoc.cuh:269-282). First
@@ -1037,7 +994,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
         for (int k = 0; k < K; ++k) {
             if (!((pending >> k) & 1u) || err) continue;
             unsigned long long dt = 0;
-            int r = silo_read<SLOW>(p, s.row[k], tx, pos, g.glane + k * G, dt, rec[k]);
+            int r = silo_read<SLOW, K>(p, s.row[k], tx, pos, g.glane + k * G, dt, rec[k]);
             if (r == O_DONE) { pending &= ~(1u << k); dg += dt; }
             else if (r == O_ERR) err = true;
         }
@@ -1058,7 +1015,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
     occ_lock_writes<G, SLOW, false>(p, g, s, writes, ordered, held, cts, fail, err, obst);
     bool gf = g.any(fail), ge = g.any(err);
     if (!gf && !ge) {
-        fence_acq_rel();
+        if (SLOW) fence_acq_rel();  // (the fast variant's lock RMWs are acquire operations)
         // Serialization point: write set locked (by every lane), read set not
         // yet validated (by any lane); the warp syncs order the leader's
         // sequence number between the two.
@@ -1093,7 +1050,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
     if (p.write_mode == GCC_WRITE_ROWCOPY) g.sync();
 #pragma unroll
     for (int k = 0; k < K; ++k)
-        if ((writes >> k) & 1u) apply_write<TX::kExt>(p, s.row[k], tx, pos, g.glane + k * G, s.readmask, dg);
+        if ((writes >> k) & 1u) apply_write(p, s, s.row[k], tx, pos, g.glane + k * G, dg);
     fence_acq_rel();
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -1104,7 +1061,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
 // ===========================================================================
 // TicToc (tictoc.cuh:115-368; slow_tictoc.cuh)
 // ===========================================================================
-template <bool SLOW>
+template <bool SLOW, int K>
 GCC_D int tictoc_read(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos, uint32_t i,
                       unsigned long long &dt, unsigned long long &wts, unsigned long long &rts) {
     unsigned long long *m = p.meta + row;
@@ -1113,16 +1070,15 @@ GCC_D int tictoc_read(const KParams &p, uint32_t row, uint32_t tx, uint64_t pos,
         unsigned long long x = *(volatile unsigned long long *)m;
         int r = O_RETRY;
         if (!(x & tictoc::kLock)) {
-            read_image(p, row_ptr(p, row), tx, pos, i, dt);
+            read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
             wts = tictoc::wts(x); rts = tictoc::rts(x); r = O_DONE;
         }
         latch_release(p, row);
         return r;
     }
-    unsigned long long x1 = ld_cg(m);
+    unsigned long long x1 = ld_acquire(m);
     if (x1 & tictoc::kLock) return O_RETRY;
-    fence_acq_rel();
-    read_image(p, row_ptr(p, row), tx, pos, i, dt);
+    read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
     fence_acq_rel();
     if (ld_cg(m) != x1) return O_RETRY;
     wts = tictoc::wts(x1);
@@ -1173,7 +1129,7 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
         for (int k = 0; k < K; ++k) {
             if (!((pending >> k) & 1u) || err) continue;
             unsigned long long dt = 0;
-            int r = tictoc_read<SLOW>(p, s.row[k], tx, pos, g.glane + k * G, dt, rw[k], rr[k]);
+            int r = tictoc_read<SLOW, K>(p, s.row[k], tx, pos, g.glane + k * G, dt, rw[k], rr[k]);
             if (r == O_DONE) { pending &= ~(1u << k); dg += dt; }
             else if (r == O_ERR) err = true;
         }
@@ -1228,7 +1184,7 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
     if (p.write_mode == GCC_WRITE_ROWCOPY) g.sync();
 #pragma unroll
     for (int k = 0; k < K; ++k)
-        if ((writes >> k) & 1u) apply_write<TX::kExt>(p, s.row[k], tx, pos, g.glane + k * G, s.readmask, dg);
+        if ((writes >> k) & 1u) apply_write(p, s, s.row[k], tx, pos, g.glane + k * G, dg);
     fence_acq_rel();
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -1274,13 +1230,6 @@ GCC_D int attempt_ordered(const KParams &p, const Group<G> &g, const TX &s, uint
 #pragma unroll
     for (int k = 0; k < K; ++k)
         wait[k] = ((s.valid >> k) & 1u) ? __ldg(p.op_wait + pos * p.slot_ops + g.glane + k * G) : 0u;
-    // one request a lane: its write's field and value, before the wait
-    uint32_t wfield = 0;
-    unsigned long long wval = 0;
-    if (K == 1 && !rowcopy && (s.valid & ~s.isread & 1u)) {
-        wfield = write_field(p.write_seed, tx, g.glane);
-        wval = write_value(p.write_seed, tx, g.glane);
-    }
     uint32_t pending = s.valid;
     unsigned long long done_ops = 0;
     uint64_t t0 = 0;
@@ -1305,11 +1254,9 @@ GCC_D int attempt_ordered(const KParams &p, const Group<G> &g, const TX &s, uint
                 continue;
             }
             if (rd) {
-                read_image(p, row_ptr(p, s.row[k]), tx, pos, i, dg);
-            } else if (K == 1 && !rowcopy) {
-                __stcg((unsigned long long *)(row_ptr(p, s.row[k]) + 1 + wfield), wval);
+                read_image<K>(p, row_ptr(p, s.row[k]), tx, pos, i, dg);
             } else {
-                apply_write<TX::kExt>(p, s.row[k], tx, pos, i, s.readmask, dg);
+                apply_write(p, s, s.row[k], tx, pos, i, dg);
             }
             // release: this access comes before those that wait for it
             red_add_rel(p.turn + s.row[k], 1u);
@@ -1391,16 +1338,34 @@ __host__ __device__ constexpr unsigned ordered_after(int s) {
 }
 
 // ===========================================================================
-// The persistent transaction kernel.
+// The persistent transaction kernel. Without contention it is bound by the
+// round trips that follow one another in a transaction (ticket, record, index,
+// lock word, rows, release; 32 warps an SM do not cover them) and by the L2
+// requests behind them, not by DRAM (13 % of its bandwidth) or by issue slots
+// (41 %). What takes a trip or a request out of the chain pays: one 32-byte
+// load per sector, an image's loads issued together, both kinds of lock RMW in
+// flight at once, acquire RMWs instead of fences, one fence per release for
+// all lanes, the record's slots read beside its count, error and admission
+// flags in one load after the previous commit, write values hashed before
+// anything is held, sums of the metrics per warp instead of per CTA.
+// Measured, 10,485,760 rows, r 0.9, wd 5, M tx/s before -> after:
+//   theta 0.1  tpl_nw 310 -> 402, to 204 -> 261, silo 341 -> 456, tictoc 335 -> 420
+//   theta 0.6  tpl_nw 95 -> 121, tpl_wd 110 -> 148, to 91 -> 174, silo 246 -> 317
+// Tried without gain: taking the next ticket (and prefetching its record)
+// during the current transaction (-3 ... -10 %), prefetching rows to L2 while
+// their locks are on the way (-5 % on tables past the TLB's reach).
 // ===========================================================================
 template <int SCH, int G, int MO = kMaxOps>
 __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ KParams p) {
     // Block-level histogram and metric sums (flushed once at exit) keep the
     // per-thread register budget for the transaction itself.
     __shared__ unsigned s_hist[kHistBuckets];
-    __shared__ unsigned long long s_met[8];
+    __shared__ unsigned long long s_met[32][8];  // a row per warp
+    // what a group's leader keeps through an attempt: start of the transaction
+    // (clock, ns) and of the attempt (not in registers: every lane's count)
+    __shared__ unsigned long long s_begin[1024 / G][3];
     for (int i = threadIdx.x; i < kHistBuckets; i += blockDim.x) s_hist[i] = 0u;
-    if (threadIdx.x < 8) s_met[threadIdx.x] = 0ull;
+    for (int i = threadIdx.x; i < 32 * 8; i += blockDim.x) (&s_met[0][0])[i] = 0ull;
     __syncthreads();
 
     const Group<G> g;
@@ -1418,27 +1383,30 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
     // live).
     const unsigned gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     unsigned stripe = gid % kTicketStripes, tried = 0;
+    auto ticket = [&]() { return (uint32_t)atomicAdd(&p.ctr->tickets[stripe * 16], 1ull); };
+    uint2 es = make_uint2(0u, 0u);  // leader: {err, starving} after its last transaction
+    if (g.glane == 0) es = ld_err_starving(p.ctr);
     while (true) {
-        unsigned long long pos = 0;
+        uint32_t pos = 0;
         unsigned stop = 0;
         if (g.glane == 0) {
             // admission pause: while some transaction is starving (it has
-            // aborted starve_limit times), take no new transaction, so the
+            // aborted starve_limit times), start no new transaction, so the
             // contention around it drains and it commits. The pause is
             // advisory: after spin_limit_ns admissions resume regardless.
-            if (p.starve_limit && ld_volatile(&p.ctr->starving) != 0u) {
+            if (p.starve_limit && es.y != 0u) {
                 const uint64_t tw = gtimer();
-                while (ld_volatile(&p.ctr->starving) != 0u) {
-                    if (error_raised(p.ctr) || expired(tw, p.spin_limit_ns)) break;
+                while (true) {
+                    es = ld_err_starving(p.ctr);
+                    if (es.y == 0u || es.x != 0u || expired(tw, p.spin_limit_ns)) break;
                     __nanosleep(1000);
                 }
             }
-            while (true) {
-                unsigned long long t = atomicAdd(&p.ctr->tickets[stripe * 16], 1ull);
-                pos = t * kTicketStripes + stripe;
-                if (pos < p.batch_n) break;
+            pos = ticket() * kTicketStripes + stripe;
+            while (pos >= p.batch_n) {
                 if (++tried >= kTicketStripes) { stop = 1u; break; }
                 stripe = (stripe + 1) % kTicketStripes;
+                pos = ticket() * kTicketStripes + stripe;
             }
             // device queue: wait (bounded) until the position is admitted
             if (!stop && p.queue_tail) {
@@ -1452,18 +1420,28 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
                     __nanosleep(256);
                 }
             }
-            if (error_raised(p.ctr)) stop = 1u;
+            if (es.x) stop = 1u;
         }
         stop = g.bcast(stop, 0);
         if (stop) break;
         pos = g.bcast(pos, 0);
-        const uint32_t tx = p.order ? __ldg(p.order + p.batch_st + pos) : p.batch_st + (uint32_t)pos;
-        const long long c_start = clock64();
-        const uint64_t t_start = gtimer();
+        const uint32_t tx = p.order ? __ldg(p.order + p.batch_st + pos) : p.batch_st + pos;
+        unsigned long long *const sum = s_met[threadIdx.x >> 5];
+        unsigned long long *const begin = s_begin[threadIdx.x / G];
+        auto add_to = [&](int j, unsigned long long v) {
+            if (G == 32) sum[j] += v;  // the warp's only writer
+            else atomicAdd(sum + j, v);
+        };
+        if (g.glane == 0) {
+            begin[0] = (unsigned long long)clock64();
+            begin[1] = gtimer();
+        }
 
         // ---- requests and index probes --------------------------------
         TX s;
         unsigned long long n64;
+        constexpr bool kEarly = MO == kMaxOps && K <= 2;
+        int2 rq[kEarly ? K : 1];
         const gcc_ycsb_tx *T = nullptr;
         uint32_t beg = 0;
         if constexpr (MO == kMaxOps) {
@@ -1474,6 +1452,15 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
             // the copy).
             n64 = p.queue_tail ? __ldcg((const unsigned long long *)&T->request_cnt)
                                : __ldg(&T->request_cnt);
+            // the slots are there whatever the count: no wait for it (where a
+            // lane has few, so that they fit its registers)
+            if constexpr (kEarly) {
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if (g.glane + k * G < kMaxOps)
+                        rq[k] = p.queue_tail ? __ldcg((const int2 *)&T->requests[g.glane + k * G])
+                                             : __ldg((const int2 *)&T->requests[g.glane + k * G]);
+            }
         } else {
             beg = __ldg(p.tx_off + tx);
             n64 = (unsigned long long)(__ldg(p.tx_off + tx + 1) - beg);
@@ -1486,47 +1473,50 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
         s.valid = s.isread = 0;
         s.obst_op = 0;
         bool miss = false;
-        unsigned long long myreads = 0;
+        typename TX::Mask myreads = 0;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const uint32_t i = g.glane + k * G;
             s.row[k] = kNoRow;
             if (i < s.n) {
-                int2 rq;
-                if constexpr (MO == kMaxOps)
-                    rq = p.queue_tail ? __ldcg((const int2 *)&T->requests[i])
+                int2 q;
+                if constexpr (kEarly) q = rq[k];
+                else if constexpr (MO != kMaxOps) q = __ldg((const int2 *)(p.reqs + beg + i));
+                else q = p.queue_tail ? __ldcg((const int2 *)&T->requests[i])
                                       : __ldg((const int2 *)&T->requests[i]);
-                else rq = __ldg((const int2 *)(p.reqs + beg + i));
                 s.valid |= 1u << k;
-                if (rq.x > 0) { s.isread |= 1u << k; myreads |= 1ull << i; }
+                if (q.x > 0) { s.isread |= 1u << k; myreads |= (typename TX::Mask)1 << i; }
                 if constexpr (is_ordered(SCH)) {
-                    s.row[k] = __ldg(p.op_row + pos * p.slot_ops + i);
+                    s.row[k] = __ldg(p.op_row + (uint64_t)pos * p.slot_ops + i);
                 } else {
-                    s.row[k] = index_find(p, (uint32_t)rq.y);
+                    s.row[k] = index_find(p, (uint32_t)q.y);
                 }
                 miss |= s.row[k] == kNoRow;
             }
         }
         s.readmask = g.orv(myreads);
+        if (K == 1 && p.write_mode == GCC_WRITE_FIELD && (s.valid & ~s.isread & 1u)) {
+            s.wfield = write_field(p.write_seed, tx, g.glane);
+            s.wval = write_value(p.write_seed, tx, g.glane);
+        }
         if (g.any(miss)) {
             if (g.glane == 0) set_error(p.ctr, GCC_EKEY, 0);
             break;
         }
-        const long long c_after_idx = clock64();
+        if (g.glane == 0) add_to(7, (unsigned long long)clock64() - begin[0]);
 
         // ---- attempt / retry loop (benchmark/ycsb.cu:51-106) -------------
         unsigned attempts = 0;
         int st = kGiveUp;
-        Clocks ck{0, 0, 0};
-        unsigned long long dg = 0, c_abort = 0;
-        long long c_attempt = c_after_idx;
+        Clocks ck{0, 0};
+        unsigned long long dg = 0;
         bool starving = false;
         // (the caller's ordered_from applies to the schemes that switch, 2PL / TO)
         const unsigned ord_from = (p.ordered_from && ordered_after(SCH) == 16u)
                                       ? p.ordered_from - 1u : ordered_after(SCH);
         while (true) {
             dg = 0;
-            c_attempt = clock64();
+            if (g.glane == 0) begin[2] = (unsigned long long)clock64();
             st = attempt<SCH, G>(p, g, s, tx, pos, dg, ck, attempts >= ord_from);
             if (st != kAbort) break;
             ++attempts;
@@ -1575,43 +1565,45 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
             // commit rule is untouched.
             if (p.backoff_ns && attempts >= 8u)
                 __nanosleep((unsigned)(hash3(tx, attempts, 0x5ull) % p.backoff_ns));
-            c_abort += clock64() - c_attempt;
-            if (g.any(expired(t_start, 4ull * p.spin_limit_ns) || error_raised(p.ctr))) {
-                if (g.glane == 0) set_error(p.ctr, GCC_ETIMEOUT, W_RETRY);
-                st = kGiveUp;
-                break;
+            unsigned late = 0;
+            if (g.glane == 0) {
+                add_to(4, (unsigned long long)clock64() - begin[2]);
+                late = expired(begin[1], 4ull * p.spin_limit_ns) || error_raised(p.ctr);
+                if (late) set_error(p.ctr, GCC_ETIMEOUT, W_RETRY);
             }
+            if (g.bcast(late, 0)) { st = kGiveUp; break; }
         }
         if (starving && g.glane == 0) {
             atomicCAS(&p.ctr->starve_token, tx + 1u, 0u);
             atomicSub(&p.ctr->starving, 1u);
         }
         if (st == kGiveUp) break;
+        if (g.glane == 0) es = ld_err_starving(p.ctr);  // for the next one's admission
         dg = g.sum(dg);
         if (g.glane == 0) {
             const long long c_end = clock64();
             p.digest[tx] = dg;
             p.tx_aborts[tx] = attempts;
             if (attempts > 64) atomicMax(&p.ctr->max_attempts, attempts + 1u);
-            atomicAdd(&s_met[0], 1ull);
-            atomicAdd(&s_met[1], (unsigned long long)attempts);
-            atomicAdd(&s_met[2], ck.ts);
-            atomicAdd(&s_met[3], ck.wait);
-            atomicAdd(&s_met[4], c_abort);
-            atomicAdd(&s_met[5], (unsigned long long)(c_end - c_attempt));
-            atomicAdd(&s_met[6], (unsigned long long)(c_end - c_start));
-            atomicAdd(&s_met[7], (unsigned long long)(c_after_idx - c_start));
-            atomicAdd(&s_hist[hist_bucket(gtimer() - t_start)], 1u);
+            add_to(0, 1ull);
+            add_to(1, attempts);
+            if (ck.ts) add_to(2, ck.ts);
+            if (ck.wait) add_to(3, ck.wait);
+            add_to(5, (unsigned long long)c_end - begin[2]);
+            add_to(6, (unsigned long long)c_end - begin[0]);
+            atomicAdd(&s_hist[hist_bucket(gtimer() - begin[1])], 1u);
         }
     }
 
     __syncthreads();
-    if (threadIdx.x < 8 && s_met[threadIdx.x]) {
+    if (threadIdx.x < 8) {
         Counters *c = p.ctr;
+        unsigned long long sum = 0;
+        for (int w = 0; w < 32; ++w) sum += s_met[w][threadIdx.x];
         unsigned long long *dst[8] = {&c->committed, &c->aborts, &c->ts_cycles, &c->wait_cycles,
                                       &c->abort_cycles, &c->mng_cycles, &c->tot_cycles,
                                       &c->idx_cycles};
-        atomicAdd(dst[threadIdx.x], s_met[threadIdx.x]);
+        if (sum) atomicAdd(dst[threadIdx.x], sum);
     }
     for (int i = threadIdx.x; i < kHistBuckets; i += blockDim.x)
         if (s_hist[i]) atomicAdd(&p.ctr->hist[i], s_hist[i]);

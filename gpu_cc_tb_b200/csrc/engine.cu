@@ -281,6 +281,7 @@ KParams gcc_engine::base_params() const {
     p.stride = stride;
     p.words = words;
     p.wslot = wslot;
+    p.wide = words == 11u;
     p.meta = meta;
     p.latch = latch;
     p.turn = turn;

@@ -41,11 +41,10 @@ GCC_HD uint32_t write_field(uint64_t wseed, uint64_t tx, uint32_t i) {
 GCC_HD uint64_t write_value(uint64_t wseed, uint64_t tx, uint32_t i) {
     return hash3(wseed, tx, 2ull * i + 1ull);
 }
-// Read digest: sum over read ops i and row words k of mix(word, i, k), so the
-// lanes of a transaction can add their parts in any order.
-GCC_HD uint64_t digest_term(uint64_t word, uint32_t i, uint32_t k) {
-    return splitmix64(word ^ ((uint64_t)(i * 16u + k + 1u) * 0xD6E8FEB86659FD93ull));
-}
+// Read digest: sum over read ops i and row words k of
+// splitmix64(word ^ (16 i + k + 1) * kDigestStep), so the lanes of a
+// transaction can add their parts in any order.
+constexpr uint64_t kDigestStep = 0xD6E8FEB86659FD93ull;
 
 // ---------------------------------------------------------------------------
 // Packed 64-bit metadata words (one per row, separate array, L2 friendly).
@@ -103,9 +102,10 @@ struct Counters {
         tot_cycles, idx_cycles;    // clock64 sums (reference Metrics)
     unsigned long long max_rank;   // gputx
     unsigned int err;              // first error status (negative gcc code)
+    unsigned int starving;         // transactions past the starvation limit
+                                   // (beside err: one load gives both)
     unsigned int err_where;        // diagnostic: which wait gave up
     unsigned int max_attempts;     // most attempts of one transaction
-    unsigned int starving;         // transactions past the starvation limit
     unsigned int starve_token;     // 0, or 1 + tx of the starving tx that retries
     unsigned int hist[kHistBuckets];
 };
@@ -148,6 +148,7 @@ struct KParams {
     uint32_t stride;            // bytes between rows (16-byte multiple)
     uint32_t words;             // 8-byte words of row payload (11 or 13)
     uint32_t wslot;             // words per row image slot (words rounded to even)
+    uint32_t wide;              // 11-word rows on 32-byte boundaries: 32-byte loads
     int32_t write_mode;
     uint64_t write_seed;
     // CC metadata
@@ -213,27 +214,41 @@ GCC_D unsigned int ld_volatile(const unsigned int *p) {
 // the sequentially consistent fence behind __threadfence().
 GCC_D void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// Atomics with acquire / release semantics at GPU scope: the lock RMW orders
-// this lane's later accesses to the row after it (acquire) and the unlock
-// RMW orders its earlier accesses before it (release), without a standalone
-// fence.
-GCC_D unsigned long long atom_add_acq(unsigned long long *p, unsigned long long v) {
+// Atomics with acquire / release semantics at GPU scope: a lock RMW orders
+// this lane's later accesses to the row after it, a turn's release add orders
+// its earlier ones before it.
+GCC_D unsigned long long atom_or_acq(unsigned long long *p, unsigned long long v) {
     unsigned long long r;
-    asm volatile("atom.acquire.gpu.global.add.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(v) : "memory");
+    asm volatile("atom.acquire.gpu.global.or.b64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(v) : "memory");
     return r;
 }
-GCC_D unsigned long long atom_cas_acq(unsigned long long *p, unsigned long long cmp,
-                                      unsigned long long val) {
+// add ? atom.add(p, 1) : atom.cas(p, 0, excl). FLAT: both predicated, so lanes
+// of the two kinds do not wait for one another's round trip as they do on the
+// two sides of a branch.
+template <bool FLAT>
+GCC_D unsigned long long atom_lock_acq(unsigned long long *p, bool add, unsigned long long excl) {
     unsigned long long r;
-    asm volatile("atom.acquire.gpu.global.cas.b64 %0, [%1], %2, %3;"
-                 : "=l"(r) : "l"(p), "l"(cmp), "l"(val) : "memory");
+    if (FLAT) {
+        asm volatile(
+            "{\n"
+            ".reg .pred a;\n"
+            "setp.ne.u32 a, %3, 0;\n"
+            "@a atom.acquire.gpu.global.add.u64 %0, [%1], 1;\n"
+            "@!a atom.acquire.gpu.global.cas.b64 %0, [%1], 0, %2;\n"
+            "}\n"
+            : "=l"(r) : "l"(p), "l"(excl), "r"((unsigned)add) : "memory");
+    } else if (add) {
+        asm volatile("atom.acquire.gpu.global.add.u64 %0, [%1], 1;" : "=l"(r) : "l"(p) : "memory");
+    } else {
+        asm volatile("atom.acquire.gpu.global.cas.b64 %0, [%1], 0, %2;"
+                     : "=l"(r) : "l"(p), "l"(excl) : "memory");
+    }
     return r;
 }
-GCC_D void red_add_rel(unsigned long long *p, unsigned long long v) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
-}
-GCC_D void red_and_rel(unsigned long long *p, unsigned long long v) {
-    asm volatile("red.release.gpu.global.and.b64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
+GCC_D unsigned long long ld_acquire(const unsigned long long *p) {
+    unsigned long long r;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(p) : "memory");
+    return r;
 }
 GCC_D unsigned ld_acquire(const unsigned *p) {
     unsigned r;
@@ -250,25 +265,30 @@ GCC_D void set_error(Counters *c, int code, unsigned where) {
 GCC_D bool error_raised(const Counters *c) {
     return *(const volatile unsigned int *)&c->err != 0u;
 }
+// {err, starving}
+GCC_D uint2 ld_err_starving(const Counters *c) {
+    uint2 v;
+    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(&c->err) : "memory");
+    return v;
+}
+// 32 bytes (one sector) in one request, from L2 / through the read-only path.
+struct Sector { unsigned long long w[4]; };
+GCC_D Sector ld_cg32(const void *p) {
+    Sector s;
+    asm volatile("ld.global.cg.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(s.w[0]), "=l"(s.w[1]), "=l"(s.w[2]), "=l"(s.w[3]) : "l"(p) : "memory");
+    return s;
+}
+GCC_D Sector ld_nc32(const void *p) {
+    Sector s;
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(s.w[0]), "=l"(s.w[1]), "=l"(s.w[2]), "=l"(s.w[3]) : "l"(p));
+    return s;
+}
 
 // Row access: payload words as 8-byte words; rows are 16-byte aligned.
 GCC_D uint64_t *row_ptr(const KParams &p, uint32_t row) {
     return (uint64_t *)(p.table + (size_t)row * p.stride);
-}
-
-// Load the whole row payload with 16-byte L2 loads (bypassing L1 so that
-// writes by other SMs are seen). `w` receives p.words words.
-template <int MAXW>
-GCC_D void load_row(const KParams &p, uint32_t row, uint64_t (&w)[MAXW]) {
-    const ulonglong2 *src = (const ulonglong2 *)row_ptr(p, row);
-#pragma unroll
-    for (int c = 0; c < MAXW / 2; ++c) {
-        if (2 * c < (int)p.words) {
-            ulonglong2 v = __ldcg(src + c);
-            w[2 * c] = v.x;
-            w[2 * c + 1] = v.y;
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -279,8 +299,8 @@ GCC_HD uint64_t hash_bucket_of(uint32_t key, uint64_t mask) {
 }
 
 // Returns the row of `key` or kNoRow. Hash buckets are one 32-byte DRAM
-// sector (4 slots of {key, row}); a probe reads one sector with two 16-byte
-// loads, linear probing on overflow.
+// sector (4 slots of {key, row}); a probe reads one sector with one load,
+// linear probing on overflow.
 GCC_D uint32_t index_find(const KParams &p, uint32_t key) {
     if (p.index_kind == GCC_INDEX_DIRECT) {
         return (uint64_t)key < p.rows ? key : kNoRow;
@@ -288,15 +308,12 @@ GCC_D uint32_t index_find(const KParams &p, uint32_t key) {
     if (p.index_kind == GCC_INDEX_HASH) {
         uint64_t b = hash_bucket_of(key, p.hash_bucket_mask);
         for (uint64_t probe = 0; probe <= p.hash_bucket_mask; ++probe) {
-            const ulonglong2 *bk = (const ulonglong2 *)(p.hash_slots + 4 * b);
-            ulonglong2 s01 = __ldg(bk);
-            ulonglong2 s23 = __ldg(bk + 1);
-            unsigned long long s[4] = {s01.x, s01.y, s23.x, s23.y};
+            const Sector s = ld_nc32(p.hash_slots + 4 * b);
             bool empty = false;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (s[j] == ~0ull) { empty = true; continue; }
-                if ((uint32_t)s[j] == key) return (uint32_t)(s[j] >> 32);
+                if (s.w[j] == ~0ull) { empty = true; continue; }
+                if ((uint32_t)s.w[j] == key) return (uint32_t)(s.w[j] >> 32);
             }
             if (empty) return kNoRow;
             b = (b + 1) & p.hash_bucket_mask;

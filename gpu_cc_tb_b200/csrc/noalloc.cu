@@ -134,6 +134,7 @@ extern "C" int gcc_run_tpl_nw_noalloc(const gcc_ycsb_tx *txs, uint64_t n_tx, voi
     p.stride = gcc_row_stride(GCC_LAYOUT_U64X11);
     p.words = gcc_row_bytes(GCC_LAYOUT_U64X11) / 8;
     p.wslot = (p.words + 1) & ~1u;
+    p.wide = (uintptr_t)table % 32 == 0;  // the caller's table may start on any 16 bytes
     p.write_mode = GCC_WRITE_FIELD;
     p.write_seed = write_seed;
     p.meta = locks;
