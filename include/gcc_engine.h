@@ -72,9 +72,10 @@ extern "C" {
 #define GCC_F_READ_LOG 2u   /* record every read row image (parity runs) */
 #define GCC_F_NO_RESET 4u   /* keep CC metadata across batches where the
                                scheme allows it (tpl, silo, tictoc) */
-#define GCC_F_RETRY_IMMEDIATE 8u /* retry an aborted transaction at once
-                               instead of first waiting (up to 50 us) until
-                               the row that made it abort looks free */
+#define GCC_F_RETRY_IMMEDIATE 8u /* 2PL: always retry an aborted transaction at
+                               once; without it a retry first waits (up to
+                               50 us) until the row that made it abort looks
+                               free while many transactions starve */
 #define GCC_F_REQUEST_ORDER 256u /* tpl_nw, tpl_wd and to: retries that
                                visit their requests one at a time do so in
                                request order (the reference's order,
