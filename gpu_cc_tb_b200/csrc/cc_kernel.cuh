@@ -1332,27 +1332,28 @@ __host__ __device__ constexpr bool is_ordered(int s) { return s == S_GACCO || s 
 // Attempts before retries switch to one request at a time (the caller can
 // move the switch of 2PL / TO with gcc_run_params.ordered_after).
 // Retries take their requests in parallel like the first attempt: Silo and
-// TicToc always, TO and 2PL for their first 15 retries, after which they go
-// one request at a time (starting from the request that failed last time,
-// see attempt_tpl / attempt_to; in key order under GCC_F_REQUEST_ORDER, which
-// is what the measurements below used). The starvation control bounds the
-// cycles that made fully parallel retries livelock. Measured (10,485,760
-// rows, r 0.9) against ordering from the first retry: silo / tictoc +40 %
-// at theta 0.6 and +25-50 % at 0.8-0.99; TO 22.9 -> 57 M tx/s at 0.6 and
-// unchanged at 0.8-0.99; tpl_nw 58 -> 67 M at 0.6, -5 % at 0.8, unchanged
-// at 0.9-0.99 (never ordering 2PL / TO gives 98 M at 0.6 but -35 % at 0.8
-// and above). The latch variants follow their fast counterparts (ordering
-// them from the first retry made every retry 16 dependent latch round trips
-// and left slow_tpl_nw at a tenth of tpl_nw at theta 0.6). MVCC
-// retries mark their writes one row at a time from the 8th on (see
-// attempt_mvcc); the ordered schemes never abort.
+// TicToc always; 2PL for the first 15 retries, after which they go one request
+// at a time (starting from the request that failed last time, see attempt_tpl;
+// in key order under GCC_F_REQUEST_ORDER); TO until its retries go one
+// transaction at a time anyway (4 x the default starvation limit): while
+// others run, a TO attempt that visits its requests in turn meets younger
+// timestamps on every one. MVCC marks its writes one by one from the 8th retry
+// on, the ordered schemes never abort. The starvation control bounds the
+// cycles that made fully parallel retries livelock. Measured, 10,485,760 rows,
+// M tx/s, one at a time from the 16th / 31st / 61st / 131st retry / never:
+//   to      theta 0.6 r 0.5            5.1 / 4.7 / 8.7 / 42 / 40
+//           theta 0.8 r 0.9            0.9 / 0.8 / 1.0 / 3.0 / 3.0
+//           theta 0.99, 512 in flight  0.27 / 0.27 / 0.25 / 0.37 / 0.39
+//   tpl_nw  theta 0.6 r 0.5            30 / 29 / 27 / 27 / 27
+//           theta 0.8 r 0.9            8.1 / 8.0 / 7.1 / 5.1 / 4.8
+//           theta 0.99, 512 in flight  1.00 / 1.05 / 0.94 / 0.64 / 0.64
+// The latch variants keep the switch of 2PL.
 __host__ __device__ constexpr unsigned ordered_after(int s) {
-    return (s == S_SILO || s == S_TICTOC || s == S_SLOW_SILO || s == S_SLOW_TICTOC)
-               ? 0xFFFFFFFFu
-               : ((s == S_TO || s == S_TPL_NW || s == S_TPL_WD || s == S_SLOW_TO ||
-                   s == S_SLOW_TPL_NW || s == S_SLOW_TPL_WD)
-                      ? 16u
-                      : 1u);
+    return (s == S_SILO || s == S_TICTOC || s == S_SLOW_SILO || s == S_SLOW_TICTOC) ? 0xFFFFFFFFu
+           : s == S_TO                                                              ? 130u
+           : (is_tpl(s) || s == S_SLOW_TO)                                          ? 16u
+           : (s == S_MVCC || s == S_SLOW_MVCC)                                      ? 8u
+                                                                                    : 1u;
 }
 
 // ===========================================================================
@@ -1532,7 +1533,7 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
         unsigned long long dg = 0;
         bool starving = false;
         // (the caller's ordered_from applies to the schemes that switch, 2PL / TO)
-        const unsigned ord_from = (p.ordered_from && ordered_after(SCH) == 16u)
+        const unsigned ord_from = (p.ordered_from && (is_tpl(SCH) || SCH == S_TO || SCH == S_SLOW_TO))
                                       ? p.ordered_from - 1u : ordered_after(SCH);
         while (true) {
             dg = 0;
