@@ -1225,14 +1225,15 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
 // that is far from its turn sleeps in proportion, because hundreds of waiters
 // polling one word slow the very release they wait for.
 // Measured, gacco, 10,485,760 rows, theta 0.8, r 0.9, batch 65,536: 26.9 ms a
-// batch with every access taking its own turn, 3.4 ms now.
+// batch with every access taking its own turn, 3.4 ms with this hand-off, 3.0
+// ms since row images are loaded at once.
 // ===========================================================================
 constexpr unsigned kWaitChecks = 16;
 // A transaction with more than kTurnNear accesses ahead of its nearest one
-// sleeps kTurnSleepNs for each of them: about what the chain takes for one at
-// read ratio 0.9 (2.1 us for a write and the ~9 reads after it). Measured on
-// the case above, a batch: 3.8 ms at 40 ns, 3.5 at 150, 4.0 at 220; 4.2 with
-// tight polls up to 64 accesses away.
+// sleeps kTurnSleepNs for each of them: under half of what the chain takes for
+// one at read ratio 0.9 (about 4 us for a write and the ~9 reads after it).
+// Measured on the case above, a batch: 3.8 ms at 40 ns, 3.5 at 150, 4.0 at
+// 220; 4.2 with tight polls up to 64 accesses away.
 constexpr uint32_t kTurnNear = 12;
 constexpr uint32_t kTurnSleepNs = 150, kTurnSleepMaxNs = 20000;
 
