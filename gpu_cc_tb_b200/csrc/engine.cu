@@ -197,8 +197,10 @@ struct gcc_engine {
         uint64_t runs = 0;
     };
     std::map<int, std::vector<Arm>> tuner;  // batch class -> candidate configs
+    // captured batched run (GCC_F_GRAPH): valid for calls with the same key
     cudaGraphExec_t graph = nullptr;
     std::vector<uint64_t> graph_key;
+    uint64_t alloc_gen = 0;  // device buffers (re)placed so far: part of that key
     std::vector<int32_t> bstat_wd, bstat_bs;
     std::vector<double> bstat_ms;
     std::vector<uint64_t> bstat_active;
@@ -217,6 +219,7 @@ struct gcc_engine {
     }
     template <class T>
     int alloc(T **p, size_t bytes) {
+        ++alloc_gen;
         if (*p) {
             cudaFree(*p);
             *p = nullptr;
@@ -1046,9 +1049,13 @@ int gcc_run_batches(gcc_engine *e, const gcc_run_params *rp, const uint32_t *bat
     p.ver_prev = e->ver_prev;
     p.ver_data = e->ver_data;
 
-    // graph key: everything the captured work depends on
+    // graph key: everything the captured work depends on. The buffers' addresses
+    // are in it through alloc_gen: any call on the engine may replace one (more
+    // transactions, a larger batch, more stamps), and the graph's kernels would
+    // go on writing to the freed one.
     std::vector<uint64_t> key = {(uint64_t)s, (uint64_t)mode, rp->flags, rp->write_seed,
-                                 p.spin_limit_ns, p.backoff_ns, p.starve_limit, (uint64_t)e->n_var, nb};
+                                 p.spin_limit_ns, p.backoff_ns, p.starve_limit, p.ordered_from,
+                                 e->alloc_gen, (uint64_t)e->n_var, nb};
     for (uint64_t b = 0; b <= nb; ++b) key.push_back(batch_off[b]);
     for (uint64_t b = 0; b < nconf; ++b) {
         key.push_back(((uint64_t)wd[b] << 48) | ((uint64_t)bs[b] << 32) | (uint64_t)grid[b]);
