@@ -347,18 +347,23 @@ struct Clocks {
 // An attempt works through its requests in stages: the group tries every
 // request of a stage's mask (bit k: the lane's k-th) until all are done, one
 // fails, or the bounded wait runs out. All stages of an attempt go through one
-// inlined copy of `op(k)`, which returns an OpResult.
-enum OpResult : int { O_DONE = 0, O_FAIL = 1, O_RETRY = 2, O_ERR = 3 };
+// inlined copy of `op(k)`, which returns an OpResult. `pre(pending)`, if there
+// is one, goes before them: it takes requests off the mask and returns the
+// stage's state bits (2: one failed).
+enum OpResult : int { O_DONE = 0, O_FAIL = 1, O_RETRY = 2, O_ERR = 3, O_LOOKED = 4 };
 struct Waiting {
     bool any = false;
     uint64_t t0 = 0;   // first wait of the attempt
     long long clk = 0;
 };
-template <int G, int K, class OP>
+struct NoPre {
+    GCC_D uint32_t operator()(uint32_t &) const { return 0u; }
+};
+template <int G, int K, class OP, class PRE = NoPre>
 GCC_D int run_stage(const KParams &p, const Group<G> &g, uint32_t pending, Waiting &w, unsigned site,
-                    OP op) {
+                    OP op, PRE pre = PRE{}) {
     while (true) {
-        uint32_t st = 0;  // 1: pending, 2: failed, 4: error
+        uint32_t st = pre(pending);  // 1: pending, 2: failed, 4: error
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             if (!((pending >> k) & 1u) || (st & 6u)) continue;
@@ -575,13 +580,13 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
 // ===========================================================================
 // Timestamp ordering (to.cuh:104-270; slow_to.cuh:137-238)
 // ===========================================================================
-// After a row's image was read under the committed word x (wts(x) <= ts): make
-// its rts cover ts. The image is of version wts(x) as long as the word keeps
-// that wts and stays committed; another reader raising rts meanwhile does not
-// change it, so only the raise is tried again, not the read. False: a writer
-// came in.
+// After a row's image was read under the committed word x (wts(x) <= ts) and
+// the reader has fenced, so that the image's loads come before the look or the
+// raise: make its rts cover ts. The image is of version wts(x) as long as the
+// word keeps that wts and stays committed; another reader raising rts meanwhile
+// does not change it, so only the raise is tried again, not the read. False: a
+// writer came in.
 GCC_D bool rts_cover(unsigned long long *m, unsigned long long x, uint64_t ts) {
-    fence_acq_rel();  // the image's loads come before the look or the raise
     const unsigned long long wts = tso::wts(x);
     bool seen = false;  // x was read after the image
     while (!(x & tso::kUnc) && tso::wts(x) == wts) {
@@ -597,13 +602,15 @@ GCC_D bool rts_cover(unsigned long long *m, unsigned long long x, uint64_t ts) {
     }
     return false;
 }
+// A read (fast variant) is O_LOOKED, with the row's word in x, once it has the
+// image: a fence and rts_cover follow.
 template <bool SLOW, int K>
 GCC_D int to_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint64_t pos,
-                  uint32_t i, unsigned long long &dt) {
+                  uint32_t i, unsigned long long &dt, unsigned long long &x) {
     unsigned long long *m = p.meta + row;
     if (SLOW) {
         if (!latch_acquire(p, row)) return O_ERR;
-        unsigned long long x = *(volatile unsigned long long *)m;
+        x = *(volatile unsigned long long *)m;
         int r;
         if (tso::wts(x) > ts) r = O_FAIL;
         else if (x & tso::kUnc) r = O_RETRY;
@@ -616,18 +623,11 @@ GCC_D int to_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, uint
         latch_release(p, row);
         return r;
     }
-    const unsigned long long x = ld_acquire(m);
+    x = ld_acquire(m);
     if (tso::wts(x) > ts) return O_FAIL;
     if (x & tso::kUnc) return O_RETRY;  // wait for the older writer
     read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
-    if (K == 1) return rts_cover(m, x, ts) ? O_DONE : O_RETRY;
-    // (a lane with several requests keeps the short form: a fence for each of
-    // them took wd 0 from 36 to 14 M tx/s)
-    if (tso::rts(x) >= ts) {
-        fence_acq_rel();
-        return ld_cg(m) == x ? O_DONE : O_RETRY;
-    }
-    return atomicCAS(m, x, tso::make(false, ts, tso::wts(x))) == x ? O_DONE : O_RETRY;
+    return O_LOOKED;
 }
 template <bool SLOW>
 GCC_D int to_write(const KParams &p, uint32_t row, uint64_t ts, unsigned long long &prev) {
@@ -691,22 +691,68 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
     const bool split = late_i != 0xFFFFFFFFu;
     uint32_t pending = ordered && !split ? 0u : s.valid & ~late;
     const uint32_t n_seq = !ordered ? 0u : split ? 1u : s.n;
+    // A lane with several requests fences once for all its reads of a pass,
+    // between their images and the raises, and makes its marks after them; the
+    // mark of a row that it still has to read waits for that read, which would
+    // otherwise wait for the mark. (A fence for each read took wd 0 from 36 to
+    // 14 M tx/s.)
+    constexpr bool kTogether = K > 1 && !SLOW;
+    uint32_t unread = 0;  // reads that the last pass left
+    auto reads_first = [&](uint32_t &left) -> uint32_t {
+        uint32_t st = 0;
+        if constexpr (kTogether) {
+            unsigned long long x[K], dt[K];
+            uint32_t looked = 0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                if (!(((left & s.isread) >> k) & 1u) || st) continue;
+                const uint32_t i = g.glane + k * G;
+                dt[k] = 0;
+                const int q = to_read<SLOW, K>(p, s.row[k], ts, tx, pos, i, dt[k], x[k]);
+                if (q == O_LOOKED) looked |= 1u << k;
+                else if (q == O_FAIL) { st = 2u; fail_i = i; }
+            }
+            if (looked) {
+                fence_acq_rel();
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if (((looked >> k) & 1u) && rts_cover(p.meta + s.row[k], x[k], ts)) {
+                        left &= ~(1u << k);
+                        dg += dt[k];
+                    }
+            }
+            unread = left & s.isread;
+            g.sync();
+        }
+        return st;
+    };
+    auto op = [&](int k) -> int {
+        const uint32_t i = g.glane + k * G;
+        int q;
+        if ((s.isread >> k) & 1u) {
+            if (kTogether) return O_RETRY;
+            unsigned long long dt = 0, x;
+            q = to_read<SLOW, K>(p, s.row[k], ts, tx, pos, i, dt, x);
+            if (q == O_LOOKED) {
+                fence_acq_rel();
+                q = rts_cover(p.meta + s.row[k], x, ts) ? O_DONE : O_RETRY;
+            }
+            if (q == O_DONE) dg += dt;
+        } else {
+            if (kTogether && unread) {
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+                    if (((unread >> j) & 1u) && s.row[j] == s.row[k]) return O_RETRY;
+            }
+            q = to_write<SLOW>(p, s.row[k], ts, prev[k]);
+            if (q == O_DONE) wrote |= 1u << k;
+        }
+        if (q == O_FAIL) fail_i = i;
+        return q;
+    };
     int r = O_DONE;
     for (uint32_t j = 0;; ++j) {
-        r = run_stage<G, K>(p, g, pending, w, W_TO_READ, [&](int k) -> int {
-            const uint32_t i = g.glane + k * G;
-            int q;
-            if ((s.isread >> k) & 1u) {
-                unsigned long long dt = 0;
-                q = to_read<SLOW, K>(p, s.row[k], ts, tx, pos, i, dt);
-                if (q == O_DONE) dg += dt;
-            } else {
-                q = to_write<SLOW>(p, s.row[k], ts, prev[k]);
-                if (q == O_DONE) wrote |= 1u << k;
-            }
-            if (q == O_FAIL) fail_i = i;
-            return q;
-        });
+        r = run_stage<G, K>(p, g, pending, w, W_TO_READ, op, reads_first);
         if (r != O_DONE || j == n_seq) break;
         pending = only(g, split ? late_i : j) & s.valid;
     }
@@ -770,6 +816,7 @@ GCC_D int mvcc_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, ui
     } else if (tso::wts(x) <= ts) {
         read_image<K>(p, row_ptr(p, row), tx, pos, i, dt);
         if (!SLOW) {
+            fence_acq_rel();
             r = rts_cover(m, x, ts) ? O_DONE : O_RETRY;
         } else {
             if (tso::rts(x) < ts) *(volatile unsigned long long *)m = tso::make(false, ts, tso::wts(x));
