@@ -1077,12 +1077,18 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
     occ_lock_writes<G, SLOW, false>(p, g, s, writes, ordered, held, cts, fail, err, obst);
     bool gf = g.any(fail), ge = g.any(err);
     if (!gf && !ge) {
-        if (SLOW) fence_acq_rel();  // (the fast variant's lock RMWs are acquire operations)
+        if (SLOW) fence_acq_rel();
         // Serialization point: write set locked (by every lane), read set not
-        // yet validated (by any lane); the warp syncs order the leader's
-        // sequence number between the two.
+        // yet validated (by any lane). Two transactions that read what the
+        // other writes must not both miss the other's lock. The fast variant's
+        // lock RMWs are acquire operations whose old values are back, so they
+        // are performed at L2, where the looks go; that orders the locking lane
+        // only (and a vote orders nothing), the warp sync makes every lane's
+        // look come after every lane's RMW, log or no log. A fence here besides
+        // (acq_rel or sc, all lanes or one) costs a quarter: theta 0.6 310 -> 230
+        // M tx/s.
+        g.sync();
         if (p.flags & GCC_F_COMMIT_LOG) {
-            g.sync();
             if (g.glane == 0) {
                 p.commit_hi[tx] = atomicAdd(&p.ctr->seq, 1ull);
                 p.commit_lo[tx] = 0ull;

@@ -209,8 +209,9 @@ GCC_D unsigned int ld_volatile(const unsigned int *p) {
     return *(const volatile unsigned int *)p;
 }
 // Acquire/release fence at GPU scope: orders this thread's earlier memory
-// operations before its later ones, which is all the lock/timestamp
-// protocols here need (no store->load Dekker patterns), and is cheaper than
+// operations before its later ones, but not a store before a later load. The
+// one place where a protocol here needs that, Silo's write locks before its
+// look at the read words, has RMWs for stores (see attempt_silo). Cheaper than
 // the sequentially consistent fence behind __threadfence().
 GCC_D void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
