@@ -823,8 +823,10 @@ GCC_D int mvcc_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, ui
             r = O_DONE;
         }
     } else {
-        // walk the version chain to the newest version with wts <= ts
-        unsigned node = ld_cg(p.turn + row);
+        // walk the version chain to the newest version with wts <= ts; a writer
+        // may be linking a newer one meanwhile, whose fields come with the
+        // acquire of the chain's head
+        unsigned node = ld_acquire(p.turn + row);
         unsigned hops = 0;
         while (node != kNoRow && tso::wts(ld_cg(p.ver_ts + node)) > ts && hops < 0x1000000u) {
             node = ld_cg(p.ver_prev + node);
@@ -835,7 +837,8 @@ GCC_D int mvcc_read(const KParams &p, uint32_t row, uint64_t ts, uint32_t tx, ui
             r = O_ERR;
         } else {
             // versions never change once linked, and the row's committed wts is
-            // past ts already: no later write can come between
+            // past ts already: no later write can come between, so the word is
+            // not looked at again
             read_image<K>(p, p.ver_data + (size_t)node * p.wslot, tx, pos, i, dt);
             r = O_DONE;
         }
@@ -937,9 +940,11 @@ GCC_D int attempt_mvcc(const KParams &p, const Group<G> &g, const TX &s, uint32_
         // push the current base row as the version it replaces, link it,
         // then install the new base row and publish (uncommitted -> 0)
         uint32_t node = (uint32_t)(pos * p.slot_ops + i);
+        // (acquire: readers of this version reach the older ones through it)
+        const uint32_t older = ld_acquire(p.turn + row);
         copy_image(p, p.ver_data + (size_t)node * p.wslot, row_ptr(p, row));
         p.ver_ts[node] = prev[k];
-        p.ver_prev[node] = ld_cg(p.turn + row);
+        p.ver_prev[node] = older;
         fence_acq_rel();
         atomicExch(p.turn + row, node);
         apply_write(p, s, row, tx, pos, i, dg);
