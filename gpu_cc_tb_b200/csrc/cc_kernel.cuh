@@ -1433,17 +1433,26 @@ __host__ __device__ constexpr unsigned ordered_after(int s) {
 // during the current transaction (-3 ... -10 %), prefetching rows to L2 while
 // their locks are on the way (-5 % on tables past the TLB's reach).
 // ===========================================================================
+// Dynamic shared memory of a CTA: the metric sums, a row per warp, and three
+// words per group. By the launch's own size: sized for 1,024 threads they cost
+// small CTAs residency (warp_density 0, block_size 1: 7 CTAs an SM instead of
+// 32; theta 0.1 103 -> 129 M tx/s).
+inline size_t ycsb_shared_bytes(int G, int block) {
+    return (size_t)(block / 32 * 8 + block / G * 3) * sizeof(unsigned long long);
+}
+
 template <int SCH, int G, int MO = kMaxOps>
 __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ KParams p) {
     // Block-level histogram and metric sums (flushed once at exit) keep the
     // per-thread register budget for the transaction itself.
     __shared__ unsigned s_hist[kHistBuckets];
-    __shared__ unsigned long long s_met[32][8];  // a row per warp
+    extern __shared__ unsigned long long s_dyn[];  // ycsb_shared_bytes
+    unsigned long long(*const s_met)[8] = (unsigned long long(*)[8])s_dyn;  // a row per warp
     // what a group's leader keeps through an attempt: start of the transaction
     // (clock, ns) and of the attempt (not in registers: every lane's count)
-    __shared__ unsigned long long s_begin[1024 / G][3];
+    unsigned long long(*const s_begin)[3] = (unsigned long long(*)[3])(s_met + blockDim.x / 32);
     for (int i = threadIdx.x; i < kHistBuckets; i += blockDim.x) s_hist[i] = 0u;
-    for (int i = threadIdx.x; i < 32 * 8; i += blockDim.x) (&s_met[0][0])[i] = 0ull;
+    for (unsigned i = threadIdx.x; i < blockDim.x / 32 * 8; i += blockDim.x) s_dyn[i] = 0ull;
     __syncthreads();
 
     const Group<G> g;
@@ -1683,7 +1692,7 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
     if (threadIdx.x < 8) {
         Counters *c = p.ctr;
         unsigned long long sum = 0;
-        for (int w = 0; w < 32; ++w) sum += s_met[w][threadIdx.x];
+        for (unsigned w = 0; w < blockDim.x / 32; ++w) sum += s_met[w][threadIdx.x];
         unsigned long long *dst[8] = {&c->committed, &c->aborts, &c->ts_cycles, &c->wait_cycles,
                                       &c->abort_cycles, &c->mng_cycles, &c->tot_cycles,
                                       &c->idx_cycles};

@@ -8,13 +8,14 @@ namespace gcc {
 
 template <int SCH>
 cudaError_t launch_one(int G, int grid, int block, const KParams &p, cudaStream_t st) {
+    const size_t shared = ycsb_shared_bytes(G, block);
     switch (G) {
-        case 1: ycsb_kernel<SCH, 1><<<grid, block, 0, st>>>(p); break;
-        case 2: ycsb_kernel<SCH, 2><<<grid, block, 0, st>>>(p); break;
-        case 4: ycsb_kernel<SCH, 4><<<grid, block, 0, st>>>(p); break;
-        case 8: ycsb_kernel<SCH, 8><<<grid, block, 0, st>>>(p); break;
-        case 16: ycsb_kernel<SCH, 16><<<grid, block, 0, st>>>(p); break;
-        case 32: ycsb_kernel<SCH, 32><<<grid, block, 0, st>>>(p); break;
+        case 1: ycsb_kernel<SCH, 1><<<grid, block, shared, st>>>(p); break;
+        case 2: ycsb_kernel<SCH, 2><<<grid, block, shared, st>>>(p); break;
+        case 4: ycsb_kernel<SCH, 4><<<grid, block, shared, st>>>(p); break;
+        case 8: ycsb_kernel<SCH, 8><<<grid, block, shared, st>>>(p); break;
+        case 16: ycsb_kernel<SCH, 16><<<grid, block, shared, st>>>(p); break;
+        case 32: ycsb_kernel<SCH, 32><<<grid, block, shared, st>>>(p); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -22,15 +23,16 @@ cudaError_t launch_one(int G, int grid, int block, const KParams &p, cudaStream_
 
 template <int SCH>
 int occupancy_one(int G, int block) {
+    const size_t shared = ycsb_shared_bytes(G, block);
     int n = 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (G) {
-        case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 1>, block, 0); break;
-        case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 2>, block, 0); break;
-        case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 4>, block, 0); break;
-        case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 8>, block, 0); break;
-        case 16: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 16>, block, 0); break;
-        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 32>, block, 0); break;
+        case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 1>, block, shared); break;
+        case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 2>, block, shared); break;
+        case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 4>, block, shared); break;
+        case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 8>, block, shared); break;
+        case 16: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 16>, block, shared); break;
+        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 32>, block, shared); break;
         default: break;
     }
     return e == cudaSuccess ? n : -1;
@@ -39,24 +41,26 @@ int occupancy_one(int G, int block) {
 // Variable-length transactions (up to 64 requests): G in {4, 8, 16, 32}.
 template <int SCH>
 cudaError_t launch_var_one(int G, int grid, int block, const KParams &p, cudaStream_t st) {
+    const size_t shared = ycsb_shared_bytes(G, block);
     switch (G) {
-        case 4: ycsb_kernel<SCH, 4, kMaxVarOps><<<grid, block, 0, st>>>(p); break;
-        case 8: ycsb_kernel<SCH, 8, kMaxVarOps><<<grid, block, 0, st>>>(p); break;
-        case 16: ycsb_kernel<SCH, 16, kMaxVarOps><<<grid, block, 0, st>>>(p); break;
-        case 32: ycsb_kernel<SCH, 32, kMaxVarOps><<<grid, block, 0, st>>>(p); break;
+        case 4: ycsb_kernel<SCH, 4, kMaxVarOps><<<grid, block, shared, st>>>(p); break;
+        case 8: ycsb_kernel<SCH, 8, kMaxVarOps><<<grid, block, shared, st>>>(p); break;
+        case 16: ycsb_kernel<SCH, 16, kMaxVarOps><<<grid, block, shared, st>>>(p); break;
+        case 32: ycsb_kernel<SCH, 32, kMaxVarOps><<<grid, block, shared, st>>>(p); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 template <int SCH>
 int occupancy_var_one(int G, int block) {
+    const size_t shared = ycsb_shared_bytes(G, block);
     int n = 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (G) {
-        case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 4, kMaxVarOps>, block, 0); break;
-        case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 8, kMaxVarOps>, block, 0); break;
-        case 16: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 16, kMaxVarOps>, block, 0); break;
-        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 32, kMaxVarOps>, block, 0); break;
+        case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 4, kMaxVarOps>, block, shared); break;
+        case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 8, kMaxVarOps>, block, shared); break;
+        case 16: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 16, kMaxVarOps>, block, shared); break;
+        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ycsb_kernel<SCH, 32, kMaxVarOps>, block, shared); break;
         default: break;
     }
     return e == cudaSuccess ? n : -1;

@@ -48,6 +48,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;
 constexpr int kG = 32, kBlock = 1024;  // one transaction per warp, 1024-thread CTAs
+const size_t kShared = gcc::ycsb_shared_bytes(kG, kBlock);
 
 // What a call needs to know about a device, looked up once per device.
 struct DeviceSetup {
@@ -72,7 +73,7 @@ int device_setup(int dev, DeviceSetup *out) {
         }
         if (major < 10) return GCC_ENODEV;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &occ, gcc::ycsb_kernel<gcc::S_TPL_NW, kG>, kBlock, 0) != cudaSuccess || occ <= 0) {
+                &occ, gcc::ycsb_kernel<gcc::S_TPL_NW, kG>, kBlock, kShared) != cudaSuccess || occ <= 0) {
             cudaGetLastError();
             return GCC_ECUDA;
         }
@@ -150,7 +151,7 @@ extern "C" int gcc_run_tpl_nw_noalloc(const gcc_ycsb_tx *txs, uint64_t n_tx, voi
 
     const uint64_t want = (n_tx * kG + kBlock - 1) / kBlock;
     const int grid = (int)(want < (uint64_t)ds.grid_cap ? want : (uint64_t)ds.grid_cap);
-    gcc::ycsb_kernel<gcc::S_TPL_NW, kG><<<grid, kBlock, 0, st>>>(p);
+    gcc::ycsb_kernel<gcc::S_TPL_NW, kG><<<grid, kBlock, kShared, st>>>(p);
     const cudaError_t le = cudaGetLastError();
     unsigned long long host[2] = {0, 0};
     unsigned err = 0;
