@@ -289,6 +289,18 @@ GCC_D void apply_write(const KParams &p, const TX &s, uint32_t row, uint32_t tx,
 // the others' ways locked). From 2, 12, 16, 30 attempts: within 5 %; one in
 // 100: 146 at theta 0.6.
 // ---------------------------------------------------------------------------
+// Where eight or more transactions share a warp (warp_density 0 to 2) each of
+// their attempts holds up the others' instructions, and retries at once cost
+// more: they wait from the kWaitFromShared-th attempt on whoever starves.
+// 65,536 transactions, r 0.9, tpl_nw, ms at warp_density 0 / 1 / 2, always
+// waiting / only while many starve / this rule:
+//   10,485,760 rows  theta 0.5  1.5 / 0.9 / 0.6   1.4 / 0.8 / 0.5   1.5 / 0.8 / 0.55
+//                    theta 0.6  4.3 / 2.4 / 1.5   6.4 / 2.5 / 1.3   4.5 / 2.3 / 1.4
+//                    theta 0.7  21 / 11 / 6.6     45 / 24 / 9.2     22 / 12 / 7.0
+//   1,048,576 rows   theta 0.4  2.1 / 1.3 / 0.7   1.9 / 1.0 / 0.5   2.0 / 1.0 / 0.6
+//                    theta 0.6  12 / 6.2 / 3.6    30 / 14 / 5.1     12 / 6.1 / 3.6
+// (from the 6th or 16th attempt: within 10 %.)
+constexpr uint32_t kWaitFromShared = 10;
 constexpr uint32_t kWaitFrom = 6;
 constexpr uint32_t kCrowdShare = 64;
 constexpr uint64_t kObstacleWaitNs = 50000;
@@ -541,7 +553,8 @@ GCC_D int attempt_tpl(const KParams &p, const Group<G> &g, const TX &s, uint32_t
         }
         // an exclusive request waits for a free word, a shared one for the
         // exclusive holder to leave
-        if (s.attempts >= kWaitFrom && s.crowded) await_row(p, obst, tpl::kExcl, obst_x);
+        if ((s.attempts >= kWaitFrom && s.crowded) || (G <= 4 && s.attempts >= kWaitFromShared))
+            await_row(p, obst, tpl::kExcl, obst_x);
         return kAbort;
     }
     // (the fast variants' lock RMWs are acquire operations)

@@ -75,7 +75,8 @@ extern "C" {
 #define GCC_F_RETRY_IMMEDIATE 8u /* 2PL: always retry an aborted transaction at
                                once; without it a retry first waits (up to
                                50 us) until the row that made it abort looks
-                               free while many transactions starve */
+                               free while many transactions starve, and at
+                               warp_density 0-2 always from the 10th on */
 #define GCC_F_REQUEST_ORDER 256u /* tpl_nw, tpl_wd and to: retries that
                                visit their requests one at a time do so in
                                request order (the reference's order,
