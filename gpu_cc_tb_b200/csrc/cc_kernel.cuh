@@ -111,6 +111,7 @@ struct TxOps {
     // none); the next one-at-a-time attempt visits it after the others
     // (unless GCC_F_REQUEST_ORDER)
     mutable uint32_t obst_op;
+    uint32_t turn_ns;   // ordered schemes: sleep for each access ahead
     uint32_t attempts;  // aborted ones so far
     bool crowded;       // many starving transactions at the last abort (see await_row)
 };
@@ -1301,12 +1302,23 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
 // ===========================================================================
 constexpr unsigned kWaitChecks = 16;
 // A transaction with more than kTurnNear accesses ahead of its nearest one
-// sleeps kTurnSleepNs for each of them: under half of what the chain takes for
-// one at read ratio 0.9 (about 4 us for a write and the ~9 reads after it).
-// Measured on the case above, a batch: 3.8 ms at 40 ns, 3.5 at 150, 4.0 at
-// 220; 4.2 with tight polls up to 64 accesses away.
+// sleeps kTurnSleepNs for each write among them, taken as the batch's share of
+// writes: the reads between two writes run together, so the time to a turn goes
+// by the writes ahead: about 4 us for one with the reads after it. A fixed time
+// an access (150 ns) fitted read ratio 0.9 and made waiters at 0.95 and above
+// sleep past their turn. Measured, gacco, theta 0.8, a batch of 65,536, ms,
+// that / 300 / 600 / 900 ns a write:
+//   r 0.5 8.7 / 8.8 / 8.7 / 8.7, 0.8 4.65 / 4.8 / 4.7 / 4.7, 0.9 2.75 / 2.75 /
+//   2.7 / 2.65, 0.95 2.05 / 1.7 / 1.55 / 1.55, 0.98 1.65 / 1.15 / 0.95 / 0.9,
+//   0.99 1.25 / 0.95 / 0.8 / 0.75; without any sleep 19.5 at 0.5, 7.2 at 0.9.
+// (Following the pace of the turn seen by each waiter instead: 3.6 at 0.9.)
 constexpr uint32_t kTurnNear = 12;
-constexpr uint32_t kTurnSleepNs = 150, kTurnSleepMaxNs = 20000;
+constexpr uint32_t kTurnSleepNs = 900, kTurnSleepMaxNs = 20000;
+
+GCC_D uint32_t turn_sleep_ns(const Counters *c) {
+    const float reads = (float)c->acc_reads, writes = (float)c->acc_writes;
+    return writes > 0.0f ? (uint32_t)((float)kTurnSleepNs * (writes / (reads + writes))) : 0u;
+}
 
 template <int G, class TX>
 GCC_D int attempt_ordered(const KParams &p, const Group<G> &g, const TX &s, uint32_t tx,
@@ -1366,7 +1378,7 @@ GCC_D int attempt_ordered(const KParams &p, const Group<G> &g, const TX &s, uint
         }
         away = __reduce_min_sync(g.mask, away);
         if (away > kTurnNear)
-            __nanosleep(min((away - kTurnNear) * kTurnSleepNs, kTurnSleepMaxNs));
+            __nanosleep(min((away - kTurnNear) * s.turn_ns, kTurnSleepMaxNs));
         else if (G < 32)
             wait_pause();  // the warp's other groups may hold the turn
     }
@@ -1464,6 +1476,8 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
     // what a group's leader keeps through an attempt: start of the transaction
     // (clock, ns) and of the attempt (not in registers: every lane's count)
     unsigned long long(*const s_begin)[3] = (unsigned long long(*)[3])(s_met + blockDim.x / 32);
+    __shared__ uint32_t s_turn_ns;
+    if (is_ordered(SCH) && threadIdx.x == 0) s_turn_ns = turn_sleep_ns(p.ctr);
     for (int i = threadIdx.x; i < kHistBuckets; i += blockDim.x) s_hist[i] = 0u;
     for (unsigned i = threadIdx.x; i < blockDim.x / 32 * 8; i += blockDim.x) s_dyn[i] = 0ull;
     __syncthreads();
@@ -1573,6 +1587,7 @@ __global__ void __launch_bounds__(1024, 1) ycsb_kernel(const __grid_constant__ K
         s.valid = s.isread = 0;
         s.obst_op = 0;
         s.attempts = 0;
+        if (is_ordered(SCH)) s.turn_ns = s_turn_ns;
         s.crowded = false;
         bool miss = false;
         typename TX::Mask myreads = 0;

@@ -388,7 +388,7 @@ int gcc_engine::order_pass(const KParams &p, uint64_t n_pos, int) {
     uint32_t *k = acc_key[0], *v = acc_val[0];
     if ((rc = radix_sort(n_acc, rbits, &k, &v))) return rc;
     k_access_waits<<<grid1d(n_acc, kWaitTile), kWaitThreads, 0, stream>>>(k, v, n_acc, invalid,
-                                                                          op_wait, turn);
+                                                                          op_wait, turn, ctr);
     CK(cudaGetLastError());
     kernel_launches += 1;
     return GCC_OK;

@@ -101,6 +101,7 @@ struct Counters {
     unsigned long long ts_cycles, wait_cycles, abort_cycles, mng_cycles,
         tot_cycles, idx_cycles;    // clock64 sums (reference Metrics)
     unsigned long long max_rank;   // gputx
+    unsigned long long acc_reads, acc_writes;  // gacco/gputx: accesses ordered so far
     unsigned int err;              // first error status (negative gcc code)
     unsigned int starving;         // transactions past the starvation limit
                                    // (beside err: one load gives both)

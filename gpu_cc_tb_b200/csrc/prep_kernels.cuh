@@ -259,7 +259,8 @@ __global__ void k_access_build(KParams p, uint64_t n_pos, uint32_t invalid_key, 
 // first position is larger than every mark before it, so the maximum needs
 // no reset at row borders. Blocks are independent: a block whose first access
 // continues a row looks backwards for the last mark, block-wide, 1,024
-// accesses a step (one step unless a run of reads is longer than that).
+// accesses a step (one step unless a run of reads is longer than that). The
+// numbers of writes and reads go to the counters (see kTurnSleepNs).
 constexpr int kWaitThreads = 256;
 constexpr int kWaitTile = kWaitThreads * 4;
 
@@ -273,13 +274,16 @@ __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *s
                                                                const uint32_t *svals,
                                                                uint64_t n_acc,
                                                                uint32_t invalid_key,
-                                                               uint32_t *op_wait, unsigned *turn) {
+                                                               uint32_t *op_wait, unsigned *turn,
+                                                               Counters *ctr) {
     __shared__ uint32_t s_warp[kWaitThreads / 32];
+    __shared__ uint32_t s_count[2];  // the tile's writes, reads
+    if (threadIdx.x < 2) s_count[threadIdx.x] = 0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint64_t base = (uint64_t)blockIdx.x * kWaitTile;
     const uint64_t q0 = base + 4ull * threadIdx.x;
     uint32_t key[4], val[4], m[4];
-    uint32_t run = 0;
+    uint32_t run = 0, count = 0;  // count: writes | reads << 16
     uint32_t before = q0 > 0 && q0 <= n_acc ? skeys[q0 - 1] : 0u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -295,7 +299,9 @@ __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *s
         before = key[j];
         run = max(run, v);
         m[j] = run;
+        if (key[j] != invalid_key) count += (val[j] >> 31) ? 1u << 16 : 1u;
     }
+    count = __reduce_add_sync(0xFFFFFFFFu, count);
     // exclusive block-wide running maximum of the threads' maxima
     uint32_t x = run;
 #pragma unroll
@@ -304,6 +310,8 @@ __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *s
     uint32_t carry = __shfl_up_sync(0xFFFFFFFFu, x, 1);
     if (lane == 0) carry = 0;
     __syncthreads();
+    if (lane < 2 && (count >> 16 * lane & 0xFFFFu))
+        atomicAdd(&s_count[lane], count >> 16 * lane & 0xFFFFu);
     for (int w = 0; w < wid; ++w) carry = max(carry, s_warp[w]);
     // the last mark before the block, where the block starts inside a row
     if (base > 0 && base < n_acc && skeys[base - 1] == skeys[base] && skeys[base] != invalid_key) {
@@ -330,6 +338,10 @@ __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *s
         if (q < n_acc && key[j] != invalid_key)
             op_wait[val[j] & 0x7FFFFFFFu] = (val[j] >> 31) ? max(m[j], carry) : (uint32_t)q;
     }
+    __syncthreads();
+    if (threadIdx.x < 2 && s_count[threadIdx.x])
+        atomicAdd(threadIdx.x ? &ctr->acc_reads : &ctr->acc_writes,
+                  (unsigned long long)s_count[threadIdx.x]);
 }
 
 // GPUTx: f[q] = 1 where a run continues and the pair (q-1, q) is not
