@@ -172,7 +172,7 @@ struct gcc_engine {
     uint64_t ver_units = 0;
     // ordering passes
     uint32_t *acc_key[2] = {nullptr, nullptr}, *acc_val[2] = {nullptr, nullptr};
-    uint32_t *op_row = nullptr, *op_wait = nullptr, *order = nullptr, *tx_rank = nullptr;
+    uint32_t *op_row = nullptr, *op_wait = nullptr, *tile_mark = nullptr, *order = nullptr, *tx_rank = nullptr;
     uint32_t *sort_counts = nullptr;
     uint64_t acc_cap = 0, counts_cap = 0, order_cap = 0;
     std::vector<uint32_t *> scan_tmp;
@@ -254,7 +254,7 @@ gcc_engine::~gcc_engine() {
     if (dev >= 0) cudaSetDevice(dev);
     void *bufs[] = {table, hash_slots, sorted, txs, meta, latch, turn, digest, commit_hi,
                     commit_lo, tx_aborts, read_log, scratch, ver_ts, ver_prev, ver_data,
-                    acc_key[0], acc_key[1], acc_val[0], acc_val[1], op_row, op_wait, order,
+                    acc_key[0], acc_key[1], acc_val[0], acc_val[1], op_row, op_wait, tile_mark, order,
                     tx_rank, sort_counts, ctr, tx_off_d, reqs_d, queue_tail, stamps};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -368,6 +368,7 @@ int gcc_engine::ensure_access(uint64_t n_acc) {
     }
     if ((rc = alloc(&op_row, n_acc * 4))) return rc;
     if ((rc = alloc(&op_wait, n_acc * 4))) return rc;
+    if ((rc = alloc(&tile_mark, grid1d(n_acc, kWaitTile) * 4ull))) return rc;
     acc_cap = n_acc;
     return GCC_OK;
 }
@@ -387,10 +388,13 @@ int gcc_engine::order_pass(const KParams &p, uint64_t n_pos, int) {
     kernel_launches += 1;
     uint32_t *k = acc_key[0], *v = acc_val[0];
     if ((rc = radix_sort(n_acc, rbits, &k, &v))) return rc;
-    k_access_waits<<<grid1d(n_acc, kWaitTile), kWaitThreads, 0, stream>>>(k, v, n_acc, invalid,
-                                                                          op_wait, turn, ctr);
+    const unsigned tiles = grid1d(n_acc, kWaitTile);
+    k_wait_tiles<<<tiles, kWaitThreads, 0, stream>>>(k, v, n_acc, tile_mark);
     CK(cudaGetLastError());
-    kernel_launches += 1;
+    k_access_waits<<<tiles, kWaitThreads, 0, stream>>>(k, v, n_acc, invalid, tile_mark, op_wait,
+                                                       turn, ctr);
+    CK(cudaGetLastError());
+    kernel_launches += 2;
     return GCC_OK;
 }
 

@@ -257,10 +257,11 @@ __global__ void k_access_build(KParams p, uint64_t n_pos, uint32_t invalid_key, 
 // for a read (the row's first position if there is none), i.e. an inclusive
 // running maximum of {write: q + 1, first of its row: q, else 0}. A row's
 // first position is larger than every mark before it, so the maximum needs
-// no reset at row borders. Blocks are independent: a block whose first access
-// continues a row looks backwards for the last mark, block-wide, 1,024
-// accesses a step (one step unless a run of reads is longer than that). The
-// numbers of writes and reads go to the counters (see kTurnSleepNs).
+// no reset at row borders. k_wait_tiles leaves every tile's last mark; a block
+// whose first access continues a row looks backwards over those, kWaitThreads
+// tiles a step, so a row read throughout costs no more than others (over the
+// accesses themselves its blocks took quadratically many steps). The numbers of
+// writes and reads go to the counters (see kTurnSleepNs).
 constexpr int kWaitThreads = 256;
 constexpr int kWaitTile = kWaitThreads * 4;
 
@@ -270,10 +271,32 @@ __device__ __forceinline__ uint32_t wait_mark(const uint32_t *skeys, const uint3
     return (q == 0 || skeys[q - 1] != skeys[q]) ? (uint32_t)q : 0u;
 }
 
+__global__ void __launch_bounds__(kWaitThreads) k_wait_tiles(const uint32_t *skeys,
+                                                             const uint32_t *svals,
+                                                             uint64_t n_acc,
+                                                             uint32_t *tile_mark) {
+    __shared__ uint32_t s_warp[kWaitThreads / 32];
+    const uint64_t base = (uint64_t)blockIdx.x * kWaitTile;
+    uint32_t v = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t q = base + threadIdx.x + (uint64_t)j * kWaitThreads;
+        if (q < n_acc) v = max(v, wait_mark(skeys, svals, q));
+    }
+    v = __reduce_max_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kWaitThreads / 32; ++w) v = max(v, s_warp[w]);
+        tile_mark[blockIdx.x] = v;
+    }
+}
+
 __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *skeys,
                                                                const uint32_t *svals,
                                                                uint64_t n_acc,
                                                                uint32_t invalid_key,
+                                                               const uint32_t *tile_mark,
                                                                uint32_t *op_wait, unsigned *turn,
                                                                Counters *ctr) {
     __shared__ uint32_t s_warp[kWaitThreads / 32];
@@ -316,19 +339,14 @@ __global__ void __launch_bounds__(kWaitThreads) k_access_waits(const uint32_t *s
     // the last mark before the block, where the block starts inside a row
     if (base > 0 && base < n_acc && skeys[base - 1] == skeys[base] && skeys[base] != invalid_key) {
         uint32_t found = 0;
-        for (uint64_t hi = base; hi > 0 && !found;) {
+        for (uint32_t hi = blockIdx.x; hi > 0 && !found;) {
             __syncthreads();
-            uint32_t v = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint64_t back = 1ull + threadIdx.x + (uint64_t)j * kWaitThreads;
-                if (back <= hi) v = max(v, wait_mark(skeys, svals, hi - back));
-            }
-            v = __reduce_max_sync(0xFFFFFFFFu, v);
+            const uint32_t v = __reduce_max_sync(
+                0xFFFFFFFFu, threadIdx.x < hi ? tile_mark[hi - 1u - threadIdx.x] : 0u);
             if (lane == 0) s_warp[wid] = v;
             __syncthreads();
             for (int w = 0; w < kWaitThreads / 32; ++w) found = max(found, s_warp[w]);
-            hi = hi > (uint64_t)kWaitTile ? hi - kWaitTile : 0ull;
+            hi -= min(hi, (uint32_t)kWaitThreads);
         }
         carry = max(carry, found);
     }
