@@ -47,7 +47,7 @@ enum AttemptStatus : int { kCommit = 0, kAbort = 1, kGiveUp = 2 };
 // Where a bounded wait gave up (Counters::err_where).
 enum WaitSite : unsigned {
     W_LATCH = 1, W_TPL_WD, W_TO_READ, W_MVCC_READ, W_SILO_READ, W_TICTOC_READ,
-    W_TICTOC_EXT, W_TURN, W_RETRY, W_CAS, W_QUEUE, W_STARVE
+    W_TICTOC_EXT, W_TURN, W_RETRY, W_QUEUE = 11, W_STARVE
 };
 
 // ---------------------------------------------------------------------------
@@ -683,7 +683,9 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
     uint32_t fail_i = 0xFFFFFFFFu;  // request index of this lane's failed op
     // A one-at-a-time retry visits every request but one at once first and
     // then the one that failed in the previous attempt, so a contended row
-    // is held uncommitted the shortest time. Request order (the reference's)
+    // is held uncommitted the shortest time; with the default switch, which lies
+    // past the starvation limit, only where starvation control is off or the
+    // caller's ordered_after is below that limit. Request order (the reference's)
     // instead under GCC_F_REQUEST_ORDER, in the latch variant, and for a
     // starving transaction: TO's conflicts are timestamp checks, and a
     // starving transaction that reached its contended row last kept meeting
@@ -1012,55 +1014,31 @@ GCC_D int occ_lock(const KParams &p, uint32_t row, unsigned long long lockbit,
     return (cur & lockbit) ? O_FAIL : O_DONE;
 }
 
-// Lock the write set, no-wait (silo.cuh:268-281, tictoc.cuh:269-282). First
-// attempts lock in parallel; retries lock one request at a time in request
-// order. `cts` accumulates f(word before locking) over the locked words.
+// Lock the write set, no-wait and all at once (silo.cuh:268-281,
+// tictoc.cuh:269-282). `cts` accumulates f(word before locking) over the locked
+// words.
 template <int G, bool SLOW, bool TICTOC, class TX>
-GCC_D void occ_lock_writes(const KParams &p, const Group<G> &g, const TX &s,
-                           uint32_t writes, bool ordered, uint32_t &held,
-                           unsigned long long &cts, bool &fail, bool &err, uint32_t &obst) {
+GCC_D void occ_lock_writes(const KParams &p, const TX &s, uint32_t writes, uint32_t &held,
+                           unsigned long long &cts, bool &fail, bool &err) {
     constexpr int K = TX::K;
     const unsigned long long lockbit = TICTOC ? tictoc::kLock : silo::kLock;
-    if (!ordered) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (!((writes >> k) & 1u) || fail || err) continue;
-            unsigned long long cur;
-            int r = occ_lock<SLOW>(p, s.row[k], lockbit, cur);
-            if (r == O_DONE) {
-                held |= 1u << k;
-                unsigned long long c = TICTOC ? tictoc::rts(cur) + 1ull : silo::ts(cur);
-                cts = cts > c ? cts : c;
-            } else if (r == O_FAIL) { fail = true; obst = s.row[k]; }
-            else err = true;
-        }
-        return;
-    }
-    for (uint32_t i = 0; i < s.n; ++i) {
-        const int owner = (int)(i % G), kk = (int)(i / G);
-        int r = O_DONE;
-        if (g.glane == owner) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (k != kk || !((writes >> k) & 1u)) continue;
-                unsigned long long cur;
-                r = occ_lock<SLOW>(p, s.row[k], lockbit, cur);
-                if (r == O_DONE) {
-                    held |= 1u << k;
-                    unsigned long long c = TICTOC ? tictoc::rts(cur) + 1ull : silo::ts(cur);
-                    cts = cts > c ? cts : c;
-                } else if (r == O_FAIL) obst = s.row[k];
-            }
-        }
-        r = g.bcast(r, owner);
-        if (r == O_FAIL) { fail = true; break; }
-        if (r == O_ERR) { err = true; break; }
+    for (int k = 0; k < K; ++k) {
+        if (!((writes >> k) & 1u) || fail || err) continue;
+        unsigned long long cur;
+        int r = occ_lock<SLOW>(p, s.row[k], lockbit, cur);
+        if (r == O_DONE) {
+            held |= 1u << k;
+            unsigned long long c = TICTOC ? tictoc::rts(cur) + 1ull : silo::ts(cur);
+            cts = cts > c ? cts : c;
+        } else if (r == O_FAIL) fail = true;
+        else err = true;
     }
 }
 
 template <int G, bool SLOW, class TX>
 GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_t tx,
-                       uint64_t pos, unsigned long long &dg, Clocks &ck, bool ordered) {
+                       uint64_t pos, unsigned long long &dg, Clocks &ck) {
     constexpr int K = TX::K;
     unsigned long long rec[K];
     uint32_t reads = s.valid & s.isread, writes = s.valid & ~s.isread;
@@ -1092,8 +1070,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
     if (!first) ck.wait += clock64() - cw;
     // validation: lock the write set, no-wait (silo.cuh:268-281)
     unsigned long long cts = 0;
-    uint32_t obst = kNoRow;
-    occ_lock_writes<G, SLOW, false>(p, g, s, writes, ordered, held, cts, fail, err, obst);
+    occ_lock_writes<G, SLOW, false>(p, s, writes, held, cts, fail, err);
     bool gf = g.any(fail), ge = g.any(err);
     if (!gf && !ge) {
         if (SLOW) fence_acq_rel();
@@ -1118,10 +1095,7 @@ GCC_D int attempt_silo(const KParams &p, const Group<G> &g, const TX &s, uint32_
         for (int k = 0; k < K; ++k) {
             if (!((reads >> k) & 1u)) continue;
             unsigned long long x = ld_cg(p.meta + s.row[k]);
-            if (silo::ts(x) != rec[k] || (x & silo::kLock)) {
-                fail = true;
-                if (x & silo::kLock) obst = s.row[k];
-            }
+            if (silo::ts(x) != rec[k] || (x & silo::kLock)) fail = true;
             cts = cts > rec[k] ? cts : rec[k];
         }
         gf = g.any(fail);
@@ -1202,7 +1176,7 @@ GCC_D int tictoc_extend(const KParams &p, uint32_t row, unsigned long long rwts,
 
 template <int G, bool SLOW, class TX>
 GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint32_t tx,
-                         uint64_t pos, unsigned long long &dg, Clocks &ck, bool ordered) {
+                         uint64_t pos, unsigned long long &dg, Clocks &ck) {
     constexpr int K = TX::K;
     unsigned long long rw[K], rr[K];
     uint32_t reads = s.valid & s.isread, writes = s.valid & ~s.isread;
@@ -1232,8 +1206,7 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
     }
     if (!first) ck.wait += clock64() - cw;
     unsigned long long cts = 0;
-    uint32_t obst = kNoRow;
-    occ_lock_writes<G, SLOW, true>(p, g, s, writes, ordered, held, cts, fail, err, obst);
+    occ_lock_writes<G, SLOW, true>(p, s, writes, held, cts, fail, err);
     bool gf = g.any(fail), ge = g.any(err);
     if (!gf && !ge) {
 #pragma unroll
@@ -1245,7 +1218,7 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
             if (!((reads >> k) & 1u) || fail || err) continue;
             if (rr[k] >= cts) continue;
             int r = tictoc_extend<SLOW>(p, s.row[k], rw[k], cts);
-            if (r == O_FAIL) { fail = true; obst = s.row[k]; }
+            if (r == O_FAIL) fail = true;
             else if (r == O_ERR) err = true;
         }
         gf = g.any(fail);
@@ -1322,7 +1295,7 @@ GCC_D uint32_t turn_sleep_ns(const Counters *c) {
 
 template <int G, class TX>
 GCC_D int attempt_ordered(const KParams &p, const Group<G> &g, const TX &s, uint32_t tx,
-                          uint64_t pos, unsigned long long &dg, Clocks &ck, bool ordered) {
+                          uint64_t pos, unsigned long long &dg, Clocks &ck) {
     constexpr int K = TX::K;
     const bool rowcopy = p.write_mode == GCC_WRITE_ROWCOPY;
     uint32_t wait[K];
@@ -1401,11 +1374,11 @@ GCC_D int attempt(const KParams &p, const Group<G> &g, const TX &s, uint32_t tx,
     else if constexpr (SCH == S_SLOW_TO) return attempt_to<G, true>(p, g, s, tx, pos, dg, ck, ordered);
     else if constexpr (SCH == S_MVCC) return attempt_mvcc<G, false>(p, g, s, tx, pos, dg, ck, ordered);
     else if constexpr (SCH == S_SLOW_MVCC) return attempt_mvcc<G, true>(p, g, s, tx, pos, dg, ck, ordered);
-    else if constexpr (SCH == S_SILO) return attempt_silo<G, false>(p, g, s, tx, pos, dg, ck, ordered);
-    else if constexpr (SCH == S_SLOW_SILO) return attempt_silo<G, true>(p, g, s, tx, pos, dg, ck, ordered);
-    else if constexpr (SCH == S_TICTOC) return attempt_tictoc<G, false>(p, g, s, tx, pos, dg, ck, ordered);
-    else if constexpr (SCH == S_SLOW_TICTOC) return attempt_tictoc<G, true>(p, g, s, tx, pos, dg, ck, ordered);
-    else return attempt_ordered<G>(p, g, s, tx, pos, dg, ck, ordered);
+    else if constexpr (SCH == S_SILO) return attempt_silo<G, false>(p, g, s, tx, pos, dg, ck);
+    else if constexpr (SCH == S_SLOW_SILO) return attempt_silo<G, true>(p, g, s, tx, pos, dg, ck);
+    else if constexpr (SCH == S_TICTOC) return attempt_tictoc<G, false>(p, g, s, tx, pos, dg, ck);
+    else if constexpr (SCH == S_SLOW_TICTOC) return attempt_tictoc<G, true>(p, g, s, tx, pos, dg, ck);
+    else return attempt_ordered<G>(p, g, s, tx, pos, dg, ck);
 }
 
 __host__ __device__ constexpr bool is_tpl(int s) {
@@ -1418,9 +1391,10 @@ __host__ __device__ constexpr bool is_ordered(int s) { return s == S_GACCO || s 
 // Retries take their requests in parallel like the first attempt: Silo and
 // TicToc always; 2PL for the first 15 retries, after which they go one request
 // at a time (starting from the request that failed last time, see attempt_tpl;
-// in key order under GCC_F_REQUEST_ORDER); TO until its retries go one
-// transaction at a time anyway (4 x the default starvation limit): while
-// others run, a TO attempt that visits its requests in turn meets younger
+// in key order under GCC_F_REQUEST_ORDER); TO for the first 129, i.e. until its
+// retries go one transaction at a time anyway (from 4 x the default starvation
+// limit on; a caller who moves starve_limit may move ordered_after with it):
+// while others run, a TO attempt that visits its requests in turn meets younger
 // timestamps on every one. MVCC marks its writes one by one from the 8th retry
 // on, the ordered schemes never abort. The starvation control bounds the
 // cycles that made fully parallel retries livelock. Measured, 10,485,760 rows,
@@ -1445,12 +1419,13 @@ __host__ __device__ constexpr unsigned ordered_after(int s) {
 // round trips that follow one another in a transaction (ticket, record, index,
 // lock word, rows, release; 32 warps an SM do not cover them) and by the L2
 // requests behind them, not by DRAM (13 % of its bandwidth) or by issue slots
-// (41 %). What takes a trip or a request out of the chain pays: one 32-byte
-// load per sector, an image's loads issued together, both kinds of lock RMW in
-// flight at once, acquire RMWs instead of fences, one fence per release for
-// all lanes, the record's slots read beside its count, error and admission
-// flags in one load after the previous commit, write values hashed before
-// anything is held, sums of the metrics per warp instead of per CTA.
+// (41 % before the changes below). What takes a trip or a request out of the
+// chain pays: one 32-byte load per sector, an image's loads issued together,
+// both kinds of lock RMW in flight at once, acquire RMWs instead of fences, one
+// fence per release for all lanes, the record's slots read beside its count,
+// error and admission flags in one load after the previous commit, write values
+// hashed before anything is held, sums of the metrics per warp instead of per
+// CTA.
 // Measured, 10,485,760 rows, r 0.9, wd 5, M tx/s before -> after:
 //   theta 0.1  tpl_nw 310 -> 402, to 204 -> 261, silo 341 -> 456, tictoc 335 -> 420
 //   theta 0.6  tpl_nw 95 -> 121, tpl_wd 110 -> 148, to 91 -> 174, silo 246 -> 317

@@ -190,7 +190,7 @@ typedef struct gcc_run_params {
                               less. With GCC_F_AUTOTUNE the tuner picks it. */
     int32_t ordered_after; /* 2PL and TO: failed attempts after which a retry
                               visits its requests one at a time instead of
-                              all at once; 0 = 15 (to: 129) */
+                              all at once; 0 = 16 (to: 130) */
     int32_t reserved;
 } gcc_run_params;
 

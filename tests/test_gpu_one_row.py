@@ -1,6 +1,6 @@
 """The ordering pass over a row that every transaction reads: its time stays with
 that of a uniform list of the same length (looking back over the accesses one
-tile at a time took some ten times as long), and the result is the same as ever."""
+tile at a time took fifty times as long), and the result is the same as ever."""
 import numpy as np
 import pytest
 
