@@ -813,7 +813,7 @@ GCC_D int attempt_to(const KParams &p, const Group<G> &g, const TX &s, uint32_t 
 // the switch (ordered_after) mark one row at a time in request order, so two
 // writers cannot keep failing on each other's marks.
 // Measured, 10,485,760 rows, theta 0.6, r 0.5, 100,003 transactions in batches
-// of 65,536: 30.6 -> 9.5 ms a run; r 0.9, 262,144 transactions: 15.3 -> 2.3 ms;
+// of 65,536: 31 -> 11.6 ms a run; r 0.9, 262,144 transactions: 15.3 -> 2.3 ms;
 // theta 0.8, r 0.9, 65,536 transactions: 98 -> 11 ms. (The switch to one mark
 // at a time after 2, 8, 16 or 64 retries measures the same within 3 %.)
 // Two reference defects are not reproduced: the base row is updated at commit
@@ -1270,8 +1270,8 @@ GCC_D int attempt_tictoc(const KParams &p, const Group<G> &g, const TX &s, uint3
 // that is far from its turn sleeps in proportion, because hundreds of waiters
 // polling one word slow the very release they wait for.
 // Measured, gacco, 10,485,760 rows, theta 0.8, r 0.9, batch 65,536: 26.9 ms a
-// batch with every access taking its own turn, 3.4 ms with this hand-off, 3.0
-// ms since row images are loaded at once.
+// batch with every access taking its own turn, 2.65 ms now (3.4 with this
+// hand-off alone, then row images loaded at once and the sleep by writes).
 // ===========================================================================
 constexpr unsigned kWaitChecks = 16;
 // A transaction with more than kTurnNear accesses ahead of its nearest one
